@@ -295,7 +295,7 @@ orr_status orr_gl3d_step(orr_gl3d* tables, const orr_gl3d_params* params, const 
         b.nmask = t->nmask;
         b.nslot = t->nslot;
         b.wall_q = wall;
-        b.hist = outlet;
+        b.hist[0] = b.hist[1] = outlet;   // the driver's one buffer, updated in place
         b.inlet = t->inlet;
         const bool smag = params->smagorinsky_c2 > 0.0f;
         const uint32_t block = params->nx % 256 == 0 ? 256u : 128u;

@@ -621,7 +621,13 @@ struct StepBuffers3D {
     const uint32_t* nmask;   // per node, bit i: direction i bounces back (solid source)
     const int32_t* nslot;    // per node wall slot of the interpolated wall, -1 none (or null)
     const void* wall_q;      // 19 fractions per slot (arithmetic type)
-    void* hist;              // convective-outlet history (arithmetic type)
+    // Convective-outlet history (arithmetic type): a step from buffer k reads
+    // hist[k] and writes hist[1 - k] (a lattice with one buffer passes it
+    // twice).  In place, the rows that share a 32-byte sector of the history
+    // read it while their neighbours on other SMs write it, and every such
+    // read waited for the sector to come back: on the 337 x 193 x 193 binary32
+    // lattice the outlet's 37,249 nodes took 70 us of a 406 us step.
+    void* hist[2];
     const void* inlet;       // imposed inlet velocity, 3 values (arithmetic type)
 };
 
@@ -657,7 +663,7 @@ template <class S, int I, bool kSolid>
 __device__ __forceinline__ void gather_one3(const Geom3D& g, const Phys3D<typename Storage<S>::A>& p,
                                             const S* __restrict__ src, const StepBuffers3D& b,
                                             int32_t slot, uint32_t mask, int x, int y, int z,
-                                            uint64_t here,
+                                            uint64_t here, uint32_t from,
                                             typename Storage<S>::A& wall_rho,
                                             typename Storage<S>::A& out) {
     using A = typename Storage<S>::A;
@@ -721,12 +727,11 @@ __device__ __forceinline__ void gather_one3(const Geom3D& g, const Phys3D<typena
             if (g.outlet_mode == ORR_OUTLET_EXTRAPOLATION) {
                 out = up;
             } else {
-                A* hist = static_cast<A*>(b.hist);
                 const uint64_t k = static_cast<uint64_t>(d3::outlet_slot(I)) * g.ny * g.nz +
                                    static_cast<uint64_t>(y) + static_cast<uint64_t>(g.ny) * z;
                 const A u = p.outlet_speed;
-                const A v = r_div(r_add(hist[k], r_mul(u, up)), r_add(A(1), u));
-                hist[k] = v;
+                const A v = r_div(r_add(static_cast<const A*>(b.hist[from])[k], r_mul(u, up)), r_add(A(1), u));
+                static_cast<A*>(b.hist[from ^ 1u])[k] = v;
                 out = v;
             }
             return;
@@ -750,11 +755,11 @@ template <class S, int I, bool kSolid>
 __device__ __forceinline__ void gather_all3(const Geom3D& g, const Phys3D<typename Storage<S>::A>& p,
                                             const S* __restrict__ src, const StepBuffers3D& b,
                                             int32_t slot, uint32_t mask, int x, int y, int z,
-                                            uint64_t here, typename Storage<S>::A& wall_rho,
+                                            uint64_t here, uint32_t from, typename Storage<S>::A& wall_rho,
                                             typename Storage<S>::A (&f)[d3::Q]) {
     if constexpr (I < d3::Q) {
-        gather_one3<S, I, kSolid>(g, p, src, b, slot, mask, x, y, z, here, wall_rho, f[I]);
-        gather_all3<S, I + 1, kSolid>(g, p, src, b, slot, mask, x, y, z, here, wall_rho, f);
+        gather_one3<S, I, kSolid>(g, p, src, b, slot, mask, x, y, z, here, from, wall_rho, f[I]);
+        gather_all3<S, I + 1, kSolid>(g, p, src, b, slot, mask, x, y, z, here, from, wall_rho, f);
     }
 }
 
@@ -840,13 +845,14 @@ __device__ __forceinline__ void gather_flat3(const Geom3D& g, const S* __restric
 // nothing for the extrapolation outlet.
 template <class S>
 __device__ __forceinline__ void convective_blend3(const Geom3D& g, const Phys3D<typename Storage<S>::A>& p,
-                                                  const StepBuffers3D& b, uint32_t y, uint32_t z,
+                                                  const StepBuffers3D& b, uint32_t y, uint32_t z, uint32_t from,
                                                   typename Storage<S>::A (&f)[d3::Q]) {
     using A = typename Storage<S>::A;
     if (g.outlet_mode != ORR_OUTLET_CONVECTIVE) {
         return;
     }
-    A* hist = static_cast<A*>(b.hist);
+    const A* before = static_cast<const A*>(b.hist[from]);
+    A* after = static_cast<A*>(b.hist[from ^ 1u]);
     const A u = p.outlet_speed;
     const uint64_t at = static_cast<uint64_t>(y) + static_cast<uint64_t>(g.ny) * z;
     const uint64_t face = static_cast<uint64_t>(g.ny) * g.nz;
@@ -854,8 +860,8 @@ __device__ __forceinline__ void convective_blend3(const Geom3D& g, const Phys3D<
     for (int i = 0; i < d3::Q; ++i) {
         if (d3::cx(i) < 0) {
             const uint64_t k = static_cast<uint64_t>(d3::outlet_slot(i)) * face + at;
-            const A v = r_div(r_add(hist[k], r_mul(u, f[i])), r_add(A(1), u));
-            hist[k] = v;
+            const A v = r_div(r_add(before[k], r_mul(u, f[i])), r_add(A(1), u));
+            after[k] = v;
             f[i] = v;
         }
     }
@@ -870,7 +876,7 @@ __device__ __forceinline__ void convective_blend3(const Geom3D& g, const Phys3D<
 template <class S>
 __device__ __forceinline__ void bulk_edges3(const Geom3D& g, const Phys3D<typename Storage<S>::A>& p,
                                             const S* __restrict__ src, const StepBuffers3D& b,
-                                            uint32_t x, uint32_t y, uint32_t z, uint64_t here,
+                                            uint32_t x, uint32_t y, uint32_t z, uint64_t here, uint32_t from,
                                             typename Storage<S>::A (&f)[d3::Q]) {
     using A = typename Storage<S>::A;
     using T = Storage<S>;
@@ -899,7 +905,7 @@ __device__ __forceinline__ void bulk_edges3(const Geom3D& g, const Phys3D<typena
         }
     }
     if (xhi && g.x_mode == ORR_X_INFLOW_OUTFLOW) {
-        convective_blend3<S>(g, p, b, y, z, f);
+        convective_blend3<S>(g, p, b, y, z, from, f);
     }
 }
 
@@ -927,12 +933,12 @@ template <class S>
 __device__ __forceinline__ void flat_fix3(const Geom3D& g, const Phys3D<typename Storage<S>::A>& p,
                                           const S* __restrict__ src, const StepBuffers3D& b,
                                           typename Storage<S>::A (&f)[d3::Q], uint8_t cls, bool interior,
-                                          uint32_t x, uint32_t y, uint32_t z, uint64_t here) {
+                                          uint32_t x, uint32_t y, uint32_t z, uint64_t here, uint32_t from) {
     using A = typename Storage<S>::A;
     using T = Storage<S>;
     const uint64_t cells = g.cells;
     if (cls == kBulk) {
-        bulk_edges3<S>(g, p, src, b, x, y, z, here, f);
+        bulk_edges3<S>(g, p, src, b, x, y, z, here, from, f);
     } else if (interior && x != 0u && x + 1u != g.nx) {
         // Boundary node of an interior row: halfway bounce-back replaces
         // the pulls of its solid-source directions by f*_opp at the node.
@@ -947,7 +953,7 @@ __device__ __forceinline__ void flat_fix3(const Geom3D& g, const Phys3D<typename
         const uint32_t mask = cls == kBoundary ? b.nmask[here] : 0u;
         gather_flat3<S>(g, src, mask, static_cast<int>(x), static_cast<int>(y), static_cast<int>(z), here, f);
         if (x + 1u == g.nx && g.x_mode == ORR_X_INFLOW_OUTFLOW) {
-            convective_blend3<S>(g, p, b, y, z, f);
+            convective_blend3<S>(g, p, b, y, z, from, f);
         }
     }
     if (g.x_mode == ORR_X_INFLOW_OUTFLOW && x == 0u) {
@@ -963,7 +969,7 @@ __device__ __forceinline__ void flat_finish3(const Geom3D& g, const Phys3D<typen
                                              const S* __restrict__ src, S* __restrict__ dst,
                                              const StepBuffers3D& b, typename Storage<S>::A (&f)[d3::Q],
                                              uint8_t cls, bool interior, uint32_t x, uint32_t y, uint32_t z,
-                                             uint64_t here) {
+                                             uint64_t here, uint32_t from) {
     using A = typename Storage<S>::A;
     using T = Storage<S>;
     if (cls == kSolid) {
@@ -973,7 +979,7 @@ __device__ __forceinline__ void flat_finish3(const Geom3D& g, const Phys3D<typen
         }
         return;
     }
-    flat_fix3<S>(g, p, src, b, f, cls, interior, x, y, z, here);
+    flat_fix3<S>(g, p, src, b, f, cls, interior, x, y, z, here, from);
     finish3<S, kSmag>(g, p, b, f, x, y, z, here, dst);
 }
 
@@ -997,7 +1003,7 @@ template <class S, bool kSmag, bool kFlat>
 __device__ __forceinline__ void step_node3(const Geom3D& g, const Phys3D<typename Storage<S>::A>& p,
                                            const S* __restrict__ src, S* __restrict__ dst,
                                            const StepBuffers3D& b, uint32_t x, uint32_t y,
-                                           uint32_t z) {
+                                           uint32_t z, uint32_t from) {
     using A = typename Storage<S>::A;
     using T = Storage<S>;
     const uint64_t cells = g.cells;
@@ -1011,7 +1017,7 @@ __device__ __forceinline__ void step_node3(const Geom3D& g, const Phys3D<typenam
         if (interior) {
             pull3<S>(g, src, here, f);
         }
-        flat_finish3<S, kSmag>(g, p, src, dst, b, f, b.cls[here], interior, x, y, z, here);
+        flat_finish3<S, kSmag>(g, p, src, dst, b, f, b.cls[here], interior, x, y, z, here, from);
         return;
     } else {
         const uint8_t cls = b.cls[here];
@@ -1024,13 +1030,13 @@ __device__ __forceinline__ void step_node3(const Geom3D& g, const Phys3D<typenam
         }
         if (cls == kBulk) {
             pull3<S>(g, src, here, f);
-            bulk_edges3<S>(g, p, src, b, x, y, z, here, f);
+            bulk_edges3<S>(g, p, src, b, x, y, z, here, from, f);
         } else {
             const uint32_t mask = cls == kBoundary ? b.nmask[here] : 0u;
             const int32_t slot = b.nslot != nullptr ? b.nslot[here] : -1;
             A wall_rho = A(-1);
             gather_all3<S, 0, true>(g, p, src, b, slot, mask, static_cast<int>(x), static_cast<int>(y),
-                                    static_cast<int>(z), here, wall_rho, f);
+                                    static_cast<int>(z), here, from, wall_rho, f);
         }
     }
     if (g.x_mode == ORR_X_INFLOW_OUTFLOW && x == 0u) {
@@ -1056,7 +1062,7 @@ constexpr int kStepMinBlocks = sizeof(typename Storage<S>::A) == 8 ? 2
                                                                : 5;
 
 // Grid (tiles along x, ny, nz): block (t, y, z) covers x in [t B, (t + 1) B)
-// of row (y, z).
+// of row (y, z).  b.hist[0] is the source buffer's history.
 // kFlat: the lattice has g.flat set (the independent-load gather; the
 // general one otherwise).
 template <class S, bool kSmag, bool kFlat>
@@ -1067,7 +1073,7 @@ __global__ void __launch_bounds__(256, kStepMinBlocks<S, kFlat>) step3d_kernel(G
     if (x >= g.nx) {
         return;
     }
-    step_node3<S, kSmag, kFlat>(g, p, src, dst, b, x, blockIdx.y, blockIdx.z);
+    step_node3<S, kSmag, kFlat>(g, p, src, dst, b, x, blockIdx.y, blockIdx.z, 0u);
 }
 
 // Row tiles of neighbouring node pairs, for the 2-byte storage forms of a
@@ -1094,8 +1100,8 @@ __global__ void __launch_bounds__(128, kPairMinBlocks) step3d_pair_kernel(Geom3D
     const uint32_t y = blockIdx.y, z = blockIdx.z;
     if (y - 1u >= g.ny - 2u || z - 1u >= g.nz - 2u) {
         if (x0 < g.nx) {
-            step_node3<S, kSmag, true>(g, p, src, dst, b, x0, y, z);
-            step_node3<S, kSmag, true>(g, p, src, dst, b, x0 + 1u, y, z);
+            step_node3<S, kSmag, true>(g, p, src, dst, b, x0, y, z, 0u);
+            step_node3<S, kSmag, true>(g, p, src, dst, b, x0 + 1u, y, z, 0u);
         }
         return;
     }
@@ -1146,10 +1152,10 @@ __global__ void __launch_bounds__(128, kPairMinBlocks) step3d_pair_kernel(Geom3D
     }
     const uint8_t ca = static_cast<uint8_t>(cls2 & 0xffu), cb = static_cast<uint8_t>(cls2 >> 8);
     if (ca != kSolid && (ca != kBulk || x0 == 0u)) {
-        flat_fix3<S>(g, p, src, b, fa, ca, true, x0, y, z, here);
+        flat_fix3<S>(g, p, src, b, fa, ca, true, x0, y, z, here, 0u);
     }
     if (cb != kSolid && (cb != kBulk || x0 + 2u == g.nx)) {
-        flat_fix3<S>(g, p, src, b, fb, cb, true, x0 + 1u, y, z, here + 1u);
+        flat_fix3<S>(g, p, src, b, fb, cb, true, x0 + 1u, y, z, here + 1u, 0u);
     }
     float2 f[d3::Q];
 #pragma unroll

@@ -564,9 +564,10 @@ std::optional<std::size_t> memory3d(const orr_lbm3d_config& c, std::size_t links
     // Node classes (one byte), bounce-back masks, wall slots and four moment planes.
     const std::size_t slot_bytes = c.solid_wall == ORR_SOLID_INTERPOLATED ? 4 : 0;
     if (!mul(*cells, 1 + 4 + slot_bytes + 4 * a, t) || !add(total, t, total)) return std::nullopt;
-    // Outlet history.
+    // Outlet history: one copy to read and one to write for the convective outlet.
+    const std::size_t histories = c.outlet == ORR_OUTLET_CONVECTIVE ? 2 : 1;
     std::size_t face = 0;
-    if (!mul(c.ny, c.nz, face) || !mul(face, d3::kOutletSlots * a, t) || !add(total, t, total))
+    if (!mul(c.ny, c.nz, face) || !mul(face, histories * d3::kOutletSlots * a, t) || !add(total, t, total))
         return std::nullopt;
     // Wall fractions.
     if (!mul(std::max<std::size_t>(wall_slots, 1), d3::Q * a, t) || !add(total, t, total))

@@ -100,7 +100,7 @@ void initialize_state(orr_lbm3d* h, const double* rho, const double* ux, const d
     check(cudaMemcpyAsync(h->f[1], h->f[0], d3::Q * cells * h->sbytes, cudaMemcpyDeviceToDevice,
                           h->stream),
           "population copy");
-    check(h->ops->history(h->g, h->f[0], h->hist, h->stream), "history kernel");
+    check(h->ops->history(h->g, h->f[0], h->hist[0], h->stream), "history kernel");
     // The status word and the stall-request word after it.
     check(cudaMemsetAsync(h->status(), 0, 2 * sizeof(uint32_t), h->stream), "status reset");
     ++h->epoch;
@@ -265,9 +265,11 @@ orr_status orr_lbm3d_create(const orr_lbm3d_config* config, const uint8_t* solid
             if (interpolated) {
                 hp->nslot = device_alloc<int32_t>(cells, "wall slot buffer");
             }
-            check(cudaMalloc(&hp->hist,
-                             static_cast<std::size_t>(d3::kOutletSlots) * config->ny * config->nz * hp->abytes),
-                  "outlet buffer");
+            const std::size_t history =
+                static_cast<std::size_t>(d3::kOutletSlots) * config->ny * config->nz * hp->abytes;
+            const bool twice = config->outlet == ORR_OUTLET_CONVECTIVE;
+            check(cudaMalloc(&hp->hist[0], twice ? 2 * history : history), "outlet buffer");
+            hp->hist[1] = twice ? static_cast<char*>(hp->hist[0]) + history : hp->hist[0];
             check(cudaMalloc(&hp->moments, 4 * cells * hp->abytes), "moment buffer");
             check(cudaMalloc(&hp->small, 256), "small buffer");
             check(cudaMemsetAsync(hp->small, 0, 256, hp->stream), "small buffer");

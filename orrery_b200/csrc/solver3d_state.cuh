@@ -12,7 +12,8 @@
 //   wall table    19 fractions per slot (interpolated wall)
 //   links         cell, direction and fraction of every boundary link
 //   moments       4 planes (rho or rho - 1, ux, uy, uz) for read-back
-//   history       5 * ny * nz convective-outlet values
+//   history       5 * ny * nz convective-outlet values, twice (a step reads one and
+//                 writes the other; one copy for the zero-gradient outlet)
 //   small         inlet velocity (3), force/moment (6) and mass accumulators,
 //                 the persistent step's status word
 //   table         the lattice-table entry of the persistent step
@@ -126,7 +127,7 @@ struct orr_lbm3d {
     uint32_t* nmask = nullptr;
     int32_t* nslot = nullptr;
     void* wall_q = nullptr;
-    void* hist = nullptr;
+    void* hist[2] = {nullptr, nullptr}; // the history beside f[k], one allocation (the same copy twice: zero-gradient outlet)
     void* moments = nullptr;
     uint32_t* lcell = nullptr;
     uint32_t* ldir = nullptr;
@@ -149,13 +150,15 @@ struct orr_lbm3d {
     }
     double* acc() const { return reinterpret_cast<double*>(static_cast<char*>(small) + 64); }
 
-    StepBuffers3D buffers() const {
+    // The tables of a step from buffer `from` (hist[0] is its history).
+    StepBuffers3D buffers(int from = 0) const {
         StepBuffers3D b{};
         b.cls = cls;
         b.nmask = nmask;
         b.nslot = nslot;
         b.wall_q = wall_q;
-        b.hist = hist;
+        b.hist[0] = hist[from];
+        b.hist[1] = hist[1 - from];
         b.inlet = small;
         return b;
     }
@@ -168,7 +171,7 @@ struct orr_lbm3d {
         }
         if (graph) cudaGraphExecDestroy(graph);
         for (void* p : {fbase[0], fbase[1], static_cast<void*>(cls), static_cast<void*>(nmask),
-                        static_cast<void*>(nslot), wall_q, hist, moments,
+                        static_cast<void*>(nslot), wall_q, hist[0], moments,
                         static_cast<void*>(lcell), static_cast<void*>(ldir),
                         static_cast<void*>(lq), small, table}) {
             if (p) cudaFree(p);
@@ -182,7 +185,7 @@ struct orr_lbm3d {
         cls = nullptr;
         nmask = nullptr;
         nslot = nullptr;
-        wall_q = hist = moments = small = nullptr;
+        wall_q = hist[0] = hist[1] = moments = small = nullptr;
         lcell = ldir = nullptr;
         lq = nullptr;
         host_small = nullptr;
@@ -219,7 +222,7 @@ struct orr_lbm3d {
                               shape.stages, smag, shape.block, shape.npt, shape.grid, status(), stream),
                   "step kernel");
         } else {
-            check(ops->step(g, phys(), f[from], f[1 - from], buffers(), smag, block, row_npt, stream),
+            check(ops->step(g, phys(), f[from], f[1 - from], buffers(from), smag, block, row_npt, stream),
                   "step kernel");
         }
         ++launches;

@@ -221,7 +221,8 @@ template <class S, bool kSmag>
 __device__ __forceinline__ void staged_node3(const Geom3D& g, const Phys3D<typename Storage<S>::A>& p,
                                              const StepBuffers3D& b, const S* __restrict__ src,
                                              S* __restrict__ dst, typename Storage<S>::A (&f)[d3::Q],
-                                             uint8_t cls, uint32_t x, uint32_t y, uint32_t z) {
+                                             uint8_t cls, uint32_t x, uint32_t y, uint32_t z,
+                                             uint32_t from) {
     using A = typename Storage<S>::A;
     using T = Storage<S>;
     const uint64_t here = x + static_cast<uint64_t>(g.nx) * (y + static_cast<uint64_t>(g.ny) * z);
@@ -237,7 +238,7 @@ __device__ __forceinline__ void staged_node3(const Geom3D& g, const Phys3D<typen
         if (x == 0u || x + 1u == g.nx) {
             gather_flat3<S>(g, src, mask, static_cast<int>(x), static_cast<int>(y), static_cast<int>(z), here, f);
             if (x + 1u == g.nx && g.x_mode == ORR_X_INFLOW_OUTFLOW) {
-                convective_blend3<S>(g, p, b, y, z, f);
+                convective_blend3<S>(g, p, b, y, z, from, f);
             }
         } else {
             // Halfway bounce-back: the staged pull of every solid-source
@@ -250,9 +251,9 @@ __device__ __forceinline__ void staged_node3(const Geom3D& g, const Phys3D<typen
             }
         }
     } else if (x + 1u == g.nx && g.x_mode == ORR_X_INFLOW_OUTFLOW) {
-        convective_blend3<S>(g, p, b, y, z, f);
+        convective_blend3<S>(g, p, b, y, z, from, f);
     } else {
-        bulk_edges3<S>(g, p, src, b, x, y, z, here, f);
+        bulk_edges3<S>(g, p, src, b, x, y, z, here, from, f);
     }
     if (g.x_mode == ORR_X_INFLOW_OUTFLOW && x == 0u) {
         inlet_west3<A, T::kShifted>(f, static_cast<const A*>(b.inlet));
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(kStagedThreads<B>, kStagedMinBlocks<S, B>)
                 if (x < L.g.nx) {
                     const uint32_t from = L.parity ^ flip;
                     step_node3<S, kSmag, true>(L.g, L.p, static_cast<const S*>(L.f[from]),
-                                               static_cast<S*>(L.f[from ^ 1u]), L.b, x, y, z);
+                                               static_cast<S*>(L.f[from ^ 1u]), L.b, x, y, z, from);
                 }
             }
         };
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(kStagedThreads<B>, kStagedMinBlocks<S, B>)
                 }
                 if (y + 1u < L.g.ny) {
                     staged_node3<S, kSmag>(L.g, L.p, L.b, static_cast<const S*>(L.f[from]),
-                                           static_cast<S*>(L.f[from ^ 1u]), f, cls, x, y, it.w);
+                                           static_cast<S*>(L.f[from ^ 1u]), f, cls, x, y, it.w, from);
                 }
             }
             if (++s == stages) {

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kTiledThreads<B>, kTiledMinBlocks<B>)
             uint32_t y, z;
             direct_row(L.g, true, d / per_row, y, z);
             if (x < nx) {
-                step_node3<S, kSmag, true>(L.g, L.p, src, dst, L.b, x, y, z);
+                step_node3<S, kSmag, true>(L.g, L.p, src, dst, L.b, x, y, z, from);
             }
         }
         const uint32_t xx = tid % kTileW;
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kTiledThreads<B>, kTiledMinBlocks<B>)
                     for (int i = 0; i < d3::Q; ++i) {
                         f[i] = T::value(raw[p][i]);
                     }
-                    staged_node3<S, kSmag>(L.g, L.p, L.b, src, dst, f, cls[p], x, y, it.z);
+                    staged_node3<S, kSmag>(L.g, L.p, L.b, src, dst, f, cls[p], x, y, it.z, from);
                 }
             }
             if (++s == stages) {
