@@ -42,6 +42,8 @@ struct orr_gl3d {
     uint8_t* cls = nullptr;
     uint32_t* nmask = nullptr;
     int32_t* nslot = nullptr;
+    uint32_t* wall_cell = nullptr; // the boundary nodes (interpolated wall)
+    uint32_t wall_count = 0;
     float* inlet = nullptr;   // device: the imposed inlet velocity
     float inlet_host[3] = {0.0f, 0.0f, 0.0f};
     bool inlet_set = false;
@@ -50,7 +52,7 @@ struct orr_gl3d {
     ~orr_gl3d() {
         cudaSetDevice(device);
         for (void* p : {static_cast<void*>(cls), static_cast<void*>(nmask), static_cast<void*>(nslot),
-                        static_cast<void*>(inlet)}) {
+                        static_cast<void*>(wall_cell), static_cast<void*>(inlet)}) {
             if (p) cudaFree(p);
         }
     }
@@ -248,8 +250,8 @@ orr_status orr_gl3d_create(const orr_gl3d_params* params, const uint32_t* class_
         const auto open_side = [](const orr_wall& w) {
             return w.kind == ORR_WALL_PERIODIC || w.kind == ORR_WALL_SLIP;
         };
-        g.flat = open_side(c.y_low) && open_side(c.y_high) && open_side(c.z_low) && open_side(c.z_high) &&
-                 !interpolated;
+        g.open = open_side(c.y_low) && open_side(c.y_high) && open_side(c.z_low) && open_side(c.z_high);
+        g.flat = g.open && !interpolated;
         check(cudaMalloc(reinterpret_cast<void**>(&t->cls), cells + kClassPad), "gl3d class table");
         check(cudaMemsetAsync(t->cls, 0, cells + kClassPad, nullptr), "gl3d class table");
         check(cudaMalloc(reinterpret_cast<void**>(&t->nmask), cells * 4), "gl3d mask table");
@@ -259,6 +261,15 @@ orr_status orr_gl3d_create(const orr_gl3d_params* params, const uint32_t* class_
         if (interpolated) {
             check(cudaMalloc(reinterpret_cast<void**>(&t->nslot), cells * 4), "gl3d slot table");
             check(cudaMemcpy(t->nslot, slot.data(), cells * 4, cudaMemcpyHostToDevice), "gl3d slot upload");
+            std::vector<uint32_t> boundary;
+            for (std::size_t k = 0; k < cells; ++k) {
+                if (plan.cls[k] == kBoundary) boundary.push_back(static_cast<uint32_t>(k));
+            }
+            t->wall_count = static_cast<uint32_t>(boundary.size());
+            check(cudaMalloc(reinterpret_cast<void**>(&t->wall_cell), std::max<std::size_t>(boundary.size(), 1) * 4),
+                  "gl3d wall table");
+            check(cudaMemcpy(t->wall_cell, boundary.data(), boundary.size() * 4, cudaMemcpyHostToDevice),
+                  "gl3d wall upload");
         }
         // The clear and the uploads ran on the legacy stream, and a copy from
         // pageable memory may return before its data lands: wait for them
@@ -295,6 +306,8 @@ orr_status orr_gl3d_step(orr_gl3d* tables, const orr_gl3d_params* params, const 
         b.nmask = t->nmask;
         b.nslot = t->nslot;
         b.wall_q = wall;
+        b.wall_cell = t->wall_cell;
+        b.wall_count = t->wall_count;
         b.hist[0] = b.hist[1] = outlet;   // the driver's one buffer, updated in place
         b.inlet = t->inlet;
         const bool smag = params->smagorinsky_c2 > 0.0f;

@@ -41,7 +41,16 @@ struct Geom3D {
     // periodic or free-slip, halfway solid walls (gather_flat3 then serves
     // face and boundary nodes).
     int32_t flat;
+    // Open sides (periodic or free-slip y and z), whatever the solid walls;
+    // flat is open with halfway walls.
+    int32_t open;
 };
+
+// The node code a step kernel is compiled for.  General: any side and wall,
+// one direction at a time.  Halfway / Interpolated: open sides, plain pulls
+// issued with the class byte, then the wall and edge rules of the few nodes
+// that have any.
+enum class Walls { General, Halfway, Interpolated };
 
 // Real parameters in the arithmetic type (binary32 parameters are the
 // binary32 roundings of the configuration, as a Float32Uniform delivers them,
@@ -621,6 +630,9 @@ struct StepBuffers3D {
     const uint32_t* nmask;   // per node, bit i: direction i bounces back (solid source)
     const int32_t* nslot;    // per node wall slot of the interpolated wall, -1 none (or null)
     const void* wall_q;      // 19 fractions per slot (arithmetic type)
+    const uint32_t* wall_cell; // the boundary nodes (open lattices with interpolated walls)
+    uint32_t wall_count;     // their number
+    uint32_t wall_layers;    // grid layers of the wall list's blocks (set by the launcher)
     // Convective-outlet history (arithmetic type): a step from buffer k reads
     // hist[k] and writes hist[1 - k] (a lattice with one buffer passes it
     // twice).  In place, the rows that share a 32-byte sector of the history
@@ -631,27 +643,26 @@ struct StepBuffers3D {
     const void* inlet;       // imposed inlet velocity, 3 values (arithmetic type)
 };
 
-// The population `here` receives from the wall of its link i (reflected,
-// lbm3d_internal.h:181-197; lbm3_reflected, glsl:164-181).
-template <class S, int I>
-__device__ __forceinline__ typename Storage<S>::A reflected3(const S* __restrict__ src,
-                                                             uint64_t cells, uint64_t here,
-                                                             int64_t farther_off,
-                                                             typename Storage<S>::A q) {
-    using A = typename Storage<S>::A;
-    using T = Storage<S>;
-    constexpr int O = d3::opposite(I);
-    const A leaving = T::load(src + static_cast<uint64_t>(O) * cells + here);
-    if (q == A(0.5)) {
-        return leaving;
-    }
+// The population a node receives from the wall of its link (reflected,
+// lbm3d_internal.h:181-197; lbm3_reflected, glsl:164-181): `leaving` is the
+// one it sent there, `other` the second term, f*_opp at the farther node for
+// q < 1/2 and the node's own f*_i for q > 1/2.
+template <class A> __device__ __forceinline__ A reflected3(A leaving, A other, A q) {
     const A q2 = r_mul(A(2), q);
     if (q < A(0.5)) {
-        const uint64_t farther = static_cast<uint64_t>(static_cast<int64_t>(here) + farther_off);
-        return r_add(r_mul(q2, leaving), r_mul(r_sub(A(1), q2), T::load(src + O * cells + farther)));
+        return r_add(r_mul(q2, leaving), r_mul(r_sub(A(1), q2), other));
     }
-    return r_div(r_add(leaving, r_mul(r_sub(q2, A(1)), T::load(src + static_cast<uint64_t>(I) * cells + here))),
-                 q2);
+    return r_div(r_add(leaving, r_mul(r_sub(q2, A(1)), other)), q2);
+}
+
+// Index of the second term's population of link I (see reflected3).
+template <int I>
+__device__ __forceinline__ uint64_t reflected_other3(uint32_t nx, uint32_t plane, uint64_t cells, uint64_t here,
+                                                     bool near) {
+    const int64_t farther = static_cast<int64_t>(here) + d3::cx(I) + static_cast<int64_t>(nx) * d3::cy(I) +
+                            static_cast<int64_t>(plane) * d3::cz(I);
+    return near ? static_cast<uint64_t>(d3::opposite(I)) * cells + static_cast<uint64_t>(farther)
+                : static_cast<uint64_t>(I) * cells + here;
 }
 
 // General gather of direction I at node (x, y, z) (resolve_source,
@@ -743,9 +754,9 @@ __device__ __forceinline__ void gather_one3(const Geom3D& g, const Phys3D<typena
     if (kSolid && ((mask >> I) & 1u) != 0u) {
         const A q = slot >= 0 ? static_cast<const A*>(b.wall_q)[static_cast<uint64_t>(slot) * d3::Q + I]
                               : A(0.5);
-        const int64_t farther_off = static_cast<int64_t>(CX) + static_cast<int64_t>(g.nx) * CY +
-                                    static_cast<int64_t>(g.plane) * CZ;
-        out = reflected3<S, I>(src, cells, here, farther_off, q);
+        const A leaving = T::load(src + static_cast<uint64_t>(d3::opposite(I)) * cells + here);
+        out = q == A(0.5) ? leaving
+                          : reflected3<A>(leaving, T::load(src + reflected_other3<I>(g.nx, g.plane, cells, here, q < A(0.5))), q);
         return;
     }
     out = T::load(src + static_cast<uint64_t>(dir) * cells + source);
@@ -926,7 +937,7 @@ __device__ __forceinline__ void bulk_edges3(const Geom3D& g, const Phys3D<typena
 //               gather, whose side rules are uniform along the row;
 //   boundary    a node with a solid source (bounce-back / interpolated wall):
 //               the general gather with the plan's per-node direction mask.
-// The rules of a fluid node of a flat lattice once its plain pulls are in f
+// The rules of a fluid node of an open lattice once its plain pulls are in f
 // (for an interior row; elsewhere f is filled here): x-edge, wall and outlet
 // rules and the inlet, everything before the collision.
 template <class S>
@@ -961,7 +972,7 @@ __device__ __forceinline__ void flat_fix3(const Geom3D& g, const Phys3D<typename
     }
 }
 
-// The rest of a node's step on a flat lattice once its pulls are in f (for
+// The rest of a node's step on an open lattice once its pulls are in f (for
 // an interior row; elsewhere f is filled here): class, edge and wall rules,
 // the inlet, the collision and the 19 stores.
 template <class S, bool kSmag>
@@ -999,7 +1010,7 @@ __device__ __forceinline__ void pull3(const Geom3D& g, const S* __restrict__ src
     }
 }
 
-template <class S, bool kSmag, bool kFlat>
+template <class S, bool kSmag, Walls kWalls>
 __device__ __forceinline__ void step_node3(const Geom3D& g, const Phys3D<typename Storage<S>::A>& p,
                                            const S* __restrict__ src, S* __restrict__ dst,
                                            const StepBuffers3D& b, uint32_t x, uint32_t y,
@@ -1009,7 +1020,7 @@ __device__ __forceinline__ void step_node3(const Geom3D& g, const Phys3D<typenam
     const uint64_t cells = g.cells;
     const uint64_t here = x + g.nx * (y + g.ny * z);   // below 2^32 / 19
     A f[d3::Q];
-    if constexpr (kFlat) {
+    if constexpr (kWalls != Walls::General) {
         // Interior rows: every plain pull address lies inside the lattice, so
         // the 19 pulls are issued together with the class load (no dependent
         // round trip) and then used, overridden or dropped by class.
@@ -1017,7 +1028,11 @@ __device__ __forceinline__ void step_node3(const Geom3D& g, const Phys3D<typenam
         if (interior) {
             pull3<S>(g, src, here, f);
         }
-        flat_finish3<S, kSmag>(g, p, src, dst, b, f, b.cls[here], interior, x, y, z, here, from);
+        const uint8_t cls = b.cls[here];
+        if (kWalls == Walls::Interpolated && cls == kBoundary) {
+            return; // wall_node3
+        }
+        flat_finish3<S, kSmag>(g, p, src, dst, b, f, cls, interior, x, y, z, here, from);
         return;
     } else {
         const uint8_t cls = b.cls[here];
@@ -1045,6 +1060,66 @@ __device__ __forceinline__ void step_node3(const Geom3D& g, const Phys3D<typenam
     finish3<S, kSmag>(g, p, b, f, x, y, z, here, dst);
 }
 
+// The second populations of a boundary node's interpolated links (fraction
+// q other than 1/2), all requested before any is used.
+template <class S, int I>
+__device__ __forceinline__ void load_others3(const Geom3D& g, const S* __restrict__ src,
+                                             const typename Storage<S>::A (&q)[d3::Q], uint64_t here,
+                                             typename Storage<S>::A (&other)[d3::Q]) {
+    using A = typename Storage<S>::A;
+    if constexpr (I < d3::Q) {
+        if (q[I] != A(0.5)) {
+            other[I] = Storage<S>::load(src + reflected_other3<I>(g.nx, g.plane, g.cells, here, q[I] < A(0.5)));
+        }
+        load_others3<S, I + 1>(g, src, q, here, other);
+    }
+}
+
+// The step of node k of the list of boundary nodes of an open lattice with
+// interpolated walls.  Its fractions and second populations are a chain of
+// round trips (cell, mask, fractions, populations) that the row tiles do not
+// wait for: one thread per listed node, in blocks of their own that start
+// first.  In the row tiles that chain, one link after another, held a tile's
+// block for its length: 337 x 193 x 193 binary32 sphere, 10,000 boundary
+// nodes, 347 us per step against kWallListUs here (halfway walls: 334).  The
+// few sectors that both kinds of blocks write (the list's nodes are skipped
+// by the tiles) are joined in L2.
+template <class S, bool kSmag>
+__device__ __forceinline__ void wall_node3(const Geom3D& g, const Phys3D<typename Storage<S>::A>& p,
+                                           const S* __restrict__ src, S* __restrict__ dst, const StepBuffers3D& b,
+                                           uint32_t k, uint32_t from) {
+    using A = typename Storage<S>::A;
+    using T = Storage<S>;
+    const uint32_t here = b.wall_cell[k];
+    const int32_t slot = b.nslot[here];
+    const uint32_t mask = b.nmask[here];
+    const uint32_t links = slot >= 0 ? mask : 0u;   // links with a fraction of their own
+    const A* wall = static_cast<const A*>(b.wall_q) + static_cast<int64_t>(slot) * d3::Q;
+    A q[d3::Q], f[d3::Q], other[d3::Q];
+#pragma unroll
+    for (int i = 1; i < d3::Q; ++i) {
+        q[i] = (links >> i) & 1u ? wall[i] : A(0.5);
+    }
+    const uint32_t row = here / g.nx, x = here - row * g.nx, z = row / g.ny, y = row - z * g.ny;
+    gather_flat3<S>(g, src, mask, static_cast<int>(x), static_cast<int>(y), static_cast<int>(z), here, f);
+    load_others3<S, 1>(g, src, q, here, other);
+#pragma unroll
+    for (int i = 1; i < d3::Q; ++i) {
+        if (q[i] != A(0.5)) {
+            f[i] = reflected3<A>(f[i], other[i], q[i]);
+        }
+    }
+    if (g.x_mode == ORR_X_INFLOW_OUTFLOW) {
+        if (x + 1u == g.nx) {
+            convective_blend3<S>(g, p, b, y, z, from, f);
+        }
+        if (x == 0u) {
+            inlet_west3<A, T::kShifted>(f, static_cast<const A*>(b.inlet));
+        }
+    }
+    finish3<S, kSmag>(g, p, b, f, x, y, z, here, dst);
+}
+
 // Resident 256-thread blocks per SM the row step is compiled for: 48
 // registers for the binary32 flat step, 40 for the flat step of the 2-byte
 // storages, 64 for the general one, 128 for binary64.  The flat step fits 48
@@ -1055,25 +1130,37 @@ __device__ __forceinline__ void step_node3(const Geom3D& g, const Phys3D<typenam
 // gain again from 48 warps at 40 registers despite a few spilled values
 // (binary16 88.1 against 92.1 us per step, bfloat16 89.8 against 93.1);
 // binary32 loses there (105.2 against 101.1 us), so it keeps 48 registers.
-template <class S, bool kFlat>
+template <class S, Walls kWalls>
 constexpr int kStepMinBlocks = sizeof(typename Storage<S>::A) == 8 ? 2
-                               : !kFlat                        ? 4
+                               : kWalls == Walls::General      ? 4
                                : sizeof(S) == 2                ? 6
                                                                : 5;
 
 // Grid (tiles along x, ny, nz): block (t, y, z) covers x in [t B, (t + 1) B)
 // of row (y, z).  b.hist[0] is the source buffer's history.
-// kFlat: the lattice has g.flat set (the independent-load gather; the
-// general one otherwise).
-template <class S, bool kSmag, bool kFlat>
-__global__ void __launch_bounds__(256, kStepMinBlocks<S, kFlat>) step3d_kernel(Geom3D g, Phys3D<typename Storage<S>::A> p,
-                                                        const S* __restrict__ src,
-                                                        S* __restrict__ dst, StepBuffers3D b) {
+// kWalls: Halfway for lattices with g.flat set, Interpolated for those with
+// g.open only, General for the others.
+template <class S, bool kSmag, Walls kWalls>
+__global__ void __launch_bounds__(256, kStepMinBlocks<S, kWalls>)
+    step3d_kernel(Geom3D g, Phys3D<typename Storage<S>::A> p, const S* __restrict__ src, S* __restrict__ dst,
+                  StepBuffers3D b) {
+    uint32_t z = blockIdx.z;
+    if constexpr (kWalls == Walls::Interpolated) {
+        // The first wall_layers layers of the grid are the wall list's.
+        if (z < b.wall_layers) {
+            const uint32_t k = ((z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+            if (k < b.wall_count) {
+                wall_node3<S, kSmag>(g, p, src, dst, b, k, 0u);
+            }
+            return;
+        }
+        z -= b.wall_layers;
+    }
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= g.nx) {
         return;
     }
-    step_node3<S, kSmag, kFlat>(g, p, src, dst, b, x, blockIdx.y, blockIdx.z, 0u);
+    step_node3<S, kSmag, kWalls>(g, p, src, dst, b, x, blockIdx.y, z, 0u);
 }
 
 // Row tiles of neighbouring node pairs, for the 2-byte storage forms of a
@@ -1100,8 +1187,8 @@ __global__ void __launch_bounds__(128, kPairMinBlocks) step3d_pair_kernel(Geom3D
     const uint32_t y = blockIdx.y, z = blockIdx.z;
     if (y - 1u >= g.ny - 2u || z - 1u >= g.nz - 2u) {
         if (x0 < g.nx) {
-            step_node3<S, kSmag, true>(g, p, src, dst, b, x0, y, z, 0u);
-            step_node3<S, kSmag, true>(g, p, src, dst, b, x0 + 1u, y, z, 0u);
+            step_node3<S, kSmag, Walls::Halfway>(g, p, src, dst, b, x0, y, z, 0u);
+            step_node3<S, kSmag, Walls::Halfway>(g, p, src, dst, b, x0 + 1u, y, z, 0u);
         }
         return;
     }

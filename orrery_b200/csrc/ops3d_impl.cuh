@@ -34,18 +34,23 @@ template <class S> struct Launch3D {
             }
         }
         const dim3 grid(gg.tiles_x, g.ny, g.nz);
+        const auto launch = [&]<bool K>() {
+            if (g.flat) {
+                step3d_kernel<S, K, Walls::Halfway><<<grid, block, 0, s>>>(gg, p, in, out, b);
+            } else if (g.open) {
+                StepBuffers3D w = b;
+                const uint64_t layer = static_cast<uint64_t>(gg.tiles_x) * g.ny * block;
+                w.wall_layers = static_cast<uint32_t>((b.wall_count + layer - 1) / layer);
+                const dim3 with_walls(gg.tiles_x, g.ny, g.nz + w.wall_layers);
+                step3d_kernel<S, K, Walls::Interpolated><<<with_walls, block, 0, s>>>(gg, p, in, out, w);
+            } else {
+                step3d_kernel<S, K, Walls::General><<<grid, block, 0, s>>>(gg, p, in, out, b);
+            }
+        };
         if (smag) {
-            if (g.flat) {
-                step3d_kernel<S, true, true><<<grid, block, 0, s>>>(gg, p, in, out, b);
-            } else {
-                step3d_kernel<S, true, false><<<grid, block, 0, s>>>(gg, p, in, out, b);
-            }
+            launch.template operator()<true>();
         } else {
-            if (g.flat) {
-                step3d_kernel<S, false, true><<<grid, block, 0, s>>>(gg, p, in, out, b);
-            } else {
-                step3d_kernel<S, false, false><<<grid, block, 0, s>>>(gg, p, in, out, b);
-            }
+            launch.template operator()<false>();
         }
         return cudaGetLastError();
     }
@@ -114,8 +119,8 @@ template <class S> struct Launch3D {
                 return e == cudaSuccess ? a.numRegs : -1;
             }
         }
-        e = smag ? cudaFuncGetAttributes(&a, step3d_kernel<S, true, true>)
-                 : cudaFuncGetAttributes(&a, step3d_kernel<S, false, true>);
+        e = smag ? cudaFuncGetAttributes(&a, step3d_kernel<S, true, Walls::Halfway>)
+                 : cudaFuncGetAttributes(&a, step3d_kernel<S, false, Walls::Halfway>);
         return e == cudaSuccess ? a.numRegs : -1;
     }
 

@@ -540,6 +540,7 @@ Plan3D plan3d(const orr_lbm3d_config& c, const uint8_t* solid, const double* dis
         const int32_t first_slot = static_cast<int32_t>(p.wall_q.size() / d3::Q);
         for (const std::size_t h : s.slotted) {
             p.nslot[h] += first_slot;
+            p.wall_cell.push_back(static_cast<uint32_t>(h));
         }
         p.fluid += s.fluid;
         p.general += s.general;
@@ -569,8 +570,8 @@ std::optional<std::size_t> memory3d(const orr_lbm3d_config& c, std::size_t links
     std::size_t face = 0;
     if (!mul(c.ny, c.nz, face) || !mul(face, histories * d3::kOutletSlots * a, t) || !add(total, t, total))
         return std::nullopt;
-    // Wall fractions.
-    if (!mul(std::max<std::size_t>(wall_slots, 1), d3::Q * a, t) || !add(total, t, total))
+    // Wall fractions and the slots' nodes.
+    if (!mul(std::max<std::size_t>(wall_slots, 1), d3::Q * a + (c.solid_wall == ORR_SOLID_INTERPOLATED ? 4 : 0), t) || !add(total, t, total))
         return std::nullopt;
     // Links: cell, direction, fraction.
     if (!mul(links, 16, t) || !add(total, t, total)) return std::nullopt;

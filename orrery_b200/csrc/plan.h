@@ -67,6 +67,7 @@ struct Plan3D {
     CellTable<int32_t> nslot;           // per cell wall slot (interpolated wall only), -1 none
     std::size_t general = 0;            // nodes on the general gather (face + boundary)
     std::vector<double> wall_q;         // 19 fractions per slot
+    std::vector<uint32_t> wall_cell;    // the boundary node of each slot (interpolated wall only)
     std::vector<uint32_t> link_cell;    // boundary links, scan order
     std::vector<uint32_t> link_dir;
     std::vector<double> link_q;

@@ -337,8 +337,9 @@ orr_status orr_lbm3d_create(const orr_lbm3d_config* config, const uint8_t* solid
         const auto open_side = [](const orr_wall& w) {
             return w.kind == ORR_WALL_PERIODIC || w.kind == ORR_WALL_SLIP;
         };
-        g.flat = open_side(config->y_low) && open_side(config->y_high) && open_side(config->z_low) &&
-                 open_side(config->z_high) && config->solid_wall == ORR_SOLID_HALFWAY;
+        g.open = open_side(config->y_low) && open_side(config->y_high) && open_side(config->z_low) &&
+                 open_side(config->z_high);
+        g.flat = g.open && config->solid_wall == ORR_SOLID_HALFWAY;
         const bool binary32 = o.storage != ORR_STORAGE_F64;
         if (binary32) {
             g.forced = to_f32(config->body_force_x) != 0.0f || to_f32(config->body_force_y) != 0.0f ||
@@ -354,6 +355,12 @@ orr_status orr_lbm3d_create(const orr_lbm3d_config* config, const uint8_t* solid
             allocate_fixed();
         }
         check(cudaMalloc(&h->wall_q, std::max<std::size_t>(slots, 1) * d3::Q * h->abytes), "wall buffer");
+        if (interpolated) {
+            h->wall_cell = device_alloc<uint32_t>(slots, "wall buffer");
+            h->wall_count = static_cast<uint32_t>(slots);
+            check(cudaMemcpyAsync(h->wall_cell, p.wall_cell.data(), slots * 4, cudaMemcpyHostToDevice, h->stream),
+                  "wall upload");
+        }
         h->lcell = device_alloc<uint32_t>(p.link_cell.size(), "link buffer");
         h->ldir = device_alloc<uint32_t>(p.link_cell.size(), "link buffer");
         h->lq = device_alloc<double>(p.link_cell.size(), "link buffer");

@@ -9,7 +9,7 @@
 //   classes       one byte per node (solid / bulk / face / boundary), slack after
 //   masks         per node, the directions that bounce back (solid source)
 //   slots         per node, the wall-table slot (interpolated wall only)
-//   wall table    19 fractions per slot (interpolated wall)
+//   wall table    19 fractions per slot, and the boundary nodes (interpolated wall)
 //   links         cell, direction and fraction of every boundary link
 //   moments       4 planes (rho or rho - 1, ux, uy, uz) for read-back
 //   history       5 * ny * nz convective-outlet values, twice (a step reads one and
@@ -127,6 +127,8 @@ struct orr_lbm3d {
     uint32_t* nmask = nullptr;
     int32_t* nslot = nullptr;
     void* wall_q = nullptr;
+    uint32_t* wall_cell = nullptr; // the boundary nodes (interpolated wall)
+    uint32_t wall_count = 0;
     void* hist[2] = {nullptr, nullptr}; // the history beside f[k], one allocation (the same copy twice: zero-gradient outlet)
     void* moments = nullptr;
     uint32_t* lcell = nullptr;
@@ -157,6 +159,8 @@ struct orr_lbm3d {
         b.nmask = nmask;
         b.nslot = nslot;
         b.wall_q = wall_q;
+        b.wall_cell = wall_cell;
+        b.wall_count = wall_count;
         b.hist[0] = hist[from];
         b.hist[1] = hist[1 - from];
         b.inlet = small;
@@ -171,7 +175,7 @@ struct orr_lbm3d {
         }
         if (graph) cudaGraphExecDestroy(graph);
         for (void* p : {fbase[0], fbase[1], static_cast<void*>(cls), static_cast<void*>(nmask),
-                        static_cast<void*>(nslot), wall_q, hist[0], moments,
+                        static_cast<void*>(nslot), wall_q, static_cast<void*>(wall_cell), hist[0], moments,
                         static_cast<void*>(lcell), static_cast<void*>(ldir),
                         static_cast<void*>(lq), small, table}) {
             if (p) cudaFree(p);
@@ -185,6 +189,7 @@ struct orr_lbm3d {
         cls = nullptr;
         nmask = nullptr;
         nslot = nullptr;
+        wall_cell = nullptr;
         wall_q = hist[0] = hist[1] = moments = small = nullptr;
         lcell = ldir = nullptr;
         lq = nullptr;

@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kStagedThreads<B>, kStagedMinBlocks<S, B>)
                 direct_row(L.g, L.staged != 0, local / tiles, y, z);
                 if (x < L.g.nx) {
                     const uint32_t from = L.parity ^ flip;
-                    step_node3<S, kSmag, true>(L.g, L.p, static_cast<const S*>(L.f[from]),
+                    step_node3<S, kSmag, Walls::Halfway>(L.g, L.p, static_cast<const S*>(L.f[from]),
                                                static_cast<S*>(L.f[from ^ 1u]), L.b, x, y, z, from);
                 }
             }

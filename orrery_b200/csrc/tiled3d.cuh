@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kTiledThreads<B>, kTiledMinBlocks<B>)
             uint32_t y, z;
             direct_row(L.g, true, d / per_row, y, z);
             if (x < nx) {
-                step_node3<S, kSmag, true>(L.g, L.p, src, dst, L.b, x, y, z, from);
+                step_node3<S, kSmag, Walls::Halfway>(L.g, L.p, src, dst, L.b, x, y, z, from);
             }
         }
         const uint32_t xx = tid % kTileW;
