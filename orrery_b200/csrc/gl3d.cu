@@ -44,7 +44,7 @@ struct orr_gl3d {
     int32_t* nslot = nullptr;
     uint32_t* wall_cell = nullptr; // the boundary nodes (interpolated wall)
     uint32_t wall_count = 0;
-    float* inlet = nullptr;   // device: the imposed inlet velocity
+    float* inlet = nullptr;   // device: the imposed inlet velocity and absorbing targets
     float inlet_host[3] = {0.0f, 0.0f, 0.0f};
     bool inlet_set = false;
     std::string error;
@@ -176,7 +176,10 @@ void sync_inlet(orr_gl3d* t, const orr_gl3d_params& p, cudaStream_t s) {
     }
     std::memcpy(t->inlet_host, p.inlet, sizeof t->inlet_host);
     // From pageable memory: the call returns once the values are staged.
-    check(cudaMemcpyAsync(t->inlet, p.inlet, sizeof t->inlet_host, cudaMemcpyHostToDevice, s), "gl3d inlet");
+    const double v[3] = {p.inlet[0], p.inlet[1], p.inlet[2]};
+    float values[kInletValues];
+    fill_inlet(values, v);
+    check(cudaMemcpyAsync(t->inlet, values, sizeof values, cudaMemcpyHostToDevice, s), "gl3d inlet");
     t->inlet_set = true;
 }
 
@@ -255,7 +258,7 @@ orr_status orr_gl3d_create(const orr_gl3d_params* params, const uint32_t* class_
         check(cudaMalloc(reinterpret_cast<void**>(&t->cls), cells + kClassPad), "gl3d class table");
         check(cudaMemsetAsync(t->cls, 0, cells + kClassPad, nullptr), "gl3d class table");
         check(cudaMalloc(reinterpret_cast<void**>(&t->nmask), cells * 4), "gl3d mask table");
-        check(cudaMalloc(reinterpret_cast<void**>(&t->inlet), 4 * sizeof(float)), "gl3d inlet");
+        check(cudaMalloc(reinterpret_cast<void**>(&t->inlet), kInletValues * sizeof(float)), "gl3d inlet");
         check(cudaMemcpy(t->cls, plan.cls.data(), cells, cudaMemcpyHostToDevice), "gl3d class upload");
         check(cudaMemcpy(t->nmask, plan.nmask.data(), cells * 4, cudaMemcpyHostToDevice), "gl3d mask upload");
         if (interpolated) {

@@ -118,6 +118,16 @@ __device__ __forceinline__ double r_mul(double a, double b) { return a * b; }
 __device__ __forceinline__ double r_div(double a, double b) { return a / b; }
 __device__ __forceinline__ double r_fma(double a, double b, double c) { return a * b + c; }
 
+// Unfused binary64 forms of r_mul / r_sub / r_fma for the link arithmetic
+// (the binary32 ones already round explicitly); the same bits in every unit,
+// with or without FMA contraction.
+__device__ __forceinline__ float lk_mul(float a, float b) { return r_mul(a, b); }
+__device__ __forceinline__ float lk_sub(float a, float b) { return r_sub(a, b); }
+__device__ __forceinline__ float lk_fma(float a, float b, float c) { return r_fma(a, b, c); }
+__device__ __forceinline__ double lk_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double lk_sub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double lk_fma(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
+
 // Reciprocal and square root of the binary32 collision: the hardware
 // approximations refined by one Newton-Raphson step, r' = r + r (1 - x r)
 // and s' = s + (y / 2)(x - s^2) with s = x y, y ~ 1/sqrt(x), which lands
@@ -333,50 +343,88 @@ __device__ __forceinline__ void collide3(A (&f)[d3::Q], const Phys3D<A>& p, int 
 }
 
 // Relaxation rate of the absorbing layers at (x, y, z)
-// (sponge_sigma, lbm3d_internal.h:255-281; lbm3_sponge, glsl:336-353).
+// (sponge_sigma, lbm3d_internal.h:255-281; lbm3_sponge, glsl:336-353): the
+// largest of the layers' squared depths.  Depths are rounded quotients of
+// non-negative numbers, and quotient and square keep their order, so the side
+// layers (one thickness) are compared by their distances, with one division
+// for all, and only the largest depth is squared.
 template <class A>
 __device__ __forceinline__ A sponge_rate3(const Geom3D& g, const Phys3D<A>& p, uint32_t x,
                                           uint32_t y, uint32_t z) {
-    A best = 0;
-    const auto layer = [&best](uint32_t d, uint32_t t) {
+    uint32_t side = g.sponge_sides;
+    if (g.y_lo != ORR_WALL_PERIODIC) {
+        side = min(side, min(y, g.ny - 1u - y));
+    }
+    if (g.z_lo != ORR_WALL_PERIODIC) {
+        side = min(side, min(z, g.nz - 1u - z));
+    }
+    const uint32_t out = g.nx - 1u - x;
+    if (side >= g.sponge_sides && x >= g.sponge_inlet && out >= g.sponge_outlet) {
+        return A(0);
+    }
+    A depth = 0;
+    const auto layer = [&depth](uint32_t d, uint32_t t) {
         if (d < t) {
             const A r = r_div(A(t - d), A(t));
-            const A v = r_mul(r, r);
-            best = best < v ? v : best;
+            depth = depth < r ? r : depth;
         }
     };
     layer(x, g.sponge_inlet);
-    layer(g.nx - 1u - x, g.sponge_outlet);
-    if (g.y_lo != ORR_WALL_PERIODIC) {
-        layer(y, g.sponge_sides);
-        layer(g.ny - 1u - y, g.sponge_sides);
-    }
-    if (g.z_lo != ORR_WALL_PERIODIC) {
-        layer(z, g.sponge_sides);
-        layer(g.nz - 1u - z, g.sponge_sides);
-    }
-    return r_mul(p.sponge_strength, best);
+    layer(out, g.sponge_outlet);
+    layer(side, g.sponge_sides);
+    return r_mul(p.sponge_strength, r_mul(depth, depth));
 }
 
-// Absorbing-layer relaxation towards f_eq(1, u_inlet)
-// (collide tail, lbm3d_cpu.cpp:94-99; lbm3_absorb, glsl:355-368).
-template <class A, bool kShifted>
+// The imposed inlet velocity as the step reads it: 3 values, padding, and the
+// populations f_eq(1, u) (less their weights for the shifted forms) that the
+// absorbing layers relax towards.  They are the same at every node, so
+// whoever writes the velocity writes them too (absorb_target3); formed per
+// node they were 10 of the layers' 13 operations a direction.
+constexpr int kInletTargets = 4;                       // offset of the targets, in values
+constexpr int kInletValues = kInletTargets + d3::Q;
+
+// Target i (collide tail, lbm3d_cpu.cpp:94-99; lbm3_absorb, glsl:355-368).
+// Binary32 is the shifted forms' arithmetic, binary64 the unshifted one's;
+// every operation rounds on its own on host and device.
+template <class A> ORR_HD A absorb_target3(int i, const A* u) {
+    const auto mul = [](A a, A b) -> A {
+#if defined(__CUDA_ARCH__)
+        return lk_mul(a, b);
+#else
+        return a * b;
+#endif
+    };
+    const auto add = [](A a, A b) -> A {
+#if defined(__CUDA_ARCH__)
+        return lk_sub(a, -b);
+#else
+        return a + b;
+#endif
+    };
+    const A cu = add(add(mul(A(d3::cx(i)), u[0]), mul(A(d3::cy(i)), u[1])), mul(A(d3::cz(i)), u[2]));
+    const A uu = add(add(mul(u[0], u[0]), mul(u[1], u[1])), mul(u[2], u[2]));
+    if constexpr (sizeof(A) == 4) {
+        const A quad = add(mul(A(3), cu), mul(mul(A(4.5), cu), cu));
+        return mul(A(d3::w(i)), add(quad, -mul(A(1.5), uu)));
+    } else {
+        return mul(mul(A(d3::w(i)), A(1)),
+                   add(add(add(A(1), mul(A(3), cu)), mul(mul(A(4.5), cu), cu)), -mul(A(1.5), uu)));
+    }
+}
+
+// The values of `inlet` for the velocity v (host).
+template <class A> void fill_inlet(A* inlet, const double* v) {
+    for (int k = 0; k < 3; ++k) inlet[k] = static_cast<A>(v[k]);
+    inlet[3] = A(0);
+    for (int i = 0; i < d3::Q; ++i) inlet[kInletTargets + i] = absorb_target3(i, inlet);
+}
+
+// Absorbing-layer relaxation with rate s.
+template <class A>
 __device__ __forceinline__ void absorb3(A (&f)[d3::Q], A s, const A* inlet) {
-    const A ux = inlet[0], uy = inlet[1], uz = inlet[2];
 #pragma unroll
     for (int i = 0; i < d3::Q; ++i) {
-        const A cu = r_add(r_add(r_mul(A(d3::cx(i)), ux), r_mul(A(d3::cy(i)), uy)), r_mul(A(d3::cz(i)), uz));
-        const A uu = r_add(r_add(r_mul(ux, ux), r_mul(uy, uy)), r_mul(uz, uz));
-        const A quad = r_add(r_mul(A(3), cu), r_mul(r_mul(A(4.5), cu), cu));
-        A target;
-        if constexpr (kShifted) {
-            target = r_mul(A(d3::w(i)), r_sub(quad, r_mul(A(1.5), uu)));
-        } else {
-            target = r_mul(r_mul(A(d3::w(i)), A(1)),
-                           r_sub(r_add(r_add(A(1), r_mul(A(3), cu)), r_mul(r_mul(A(4.5), cu), cu)),
-                                 r_mul(A(1.5), uu)));
-        }
-        f[i] = r_sub(f[i], r_mul(s, r_sub(f[i], target)));
+        f[i] = r_sub(f[i], r_mul(s, r_sub(f[i], inlet[kInletTargets + i])));
     }
 }
 
@@ -485,16 +533,10 @@ __device__ __forceinline__ void collide3_pair(float2 (&f)[d3::Q], const Phys3D<f
 // absorb3 for two nodes with their own layer rates (a node with rate 0 keeps
 // its values, as absorb3 is then not applied to it).
 __device__ __forceinline__ void absorb3_pair(float2 (&f)[d3::Q], float sa, float sb, const float* inlet) {
-    const float ux = inlet[0], uy = inlet[1], uz = inlet[2];
     const float2 s = make_float2(sa, sb);
 #pragma unroll
     for (int i = 0; i < d3::Q; ++i) {
-        const float cu = r_add(r_add(r_mul(float(d3::cx(i)), ux), r_mul(float(d3::cy(i)), uy)),
-                               r_mul(float(d3::cz(i)), uz));
-        const float uu = r_add(r_add(r_mul(ux, ux), r_mul(uy, uy)), r_mul(uz, uz));
-        const float quad = r_add(r_mul(3.0f, cu), r_mul(r_mul(4.5f, cu), cu));
-        const float target = r_mul(float(d3::w(i)), r_sub(quad, r_mul(1.5f, uu)));
-        const float2 r = p_sub(f[i], p_mul(s, p_sub(f[i], v2(target))));
+        const float2 r = p_sub(f[i], p_mul(s, p_sub(f[i], v2(inlet[kInletTargets + i]))));
         f[i] = make_float2(sa > 0.0f ? r.x : f[i].x, sb > 0.0f ? r.y : f[i].y);
     }
 }
@@ -640,7 +682,7 @@ struct StepBuffers3D {
     // read waited for the sector to come back: on the 337 x 193 x 193 binary32
     // lattice the outlet's 37,249 nodes took 70 us of a 406 us step.
     void* hist[2];
-    const void* inlet;       // imposed inlet velocity, 3 values (arithmetic type)
+    const void* inlet;       // imposed inlet velocity and absorbing targets, kInletValues values (arithmetic type)
 };
 
 // The population a node receives from the wall of its link (reflected,
@@ -787,7 +829,7 @@ __device__ __forceinline__ void finish3(const Geom3D& g, const Phys3D<typename S
     if (g.sponge) {
         const A s = sponge_rate3<A>(g, p, x, y, z);
         if (s > A(0)) {
-            absorb3<A, T::kShifted>(f, s, static_cast<const A*>(b.inlet));
+            absorb3<A>(f, s, static_cast<const A*>(b.inlet));
         }
     }
     // Population i of the node at (dst + i * cells) + here: the first sum is
@@ -1080,8 +1122,8 @@ __device__ __forceinline__ void load_others3(const Geom3D& g, const S* __restric
 // round trips (cell, mask, fractions, populations) that the row tiles do not
 // wait for: one thread per listed node, in blocks of their own that start
 // first.  In the row tiles that chain, one link after another, held a tile's
-// block for its length: 337 x 193 x 193 binary32 sphere, 10,000 boundary
-// nodes, 347 us per step against kWallListUs here (halfway walls: 334).  The
+// block for its length: 337 x 193 x 193 binary32 sphere: 347 us per
+// step against 342 here (halfway walls: 334); 97 x 65 x 65: 20.4 against 17.5.  The
 // few sectors that both kinds of blocks write (the list's nodes are skipped
 // by the tiles) are joined in L2.
 template <class S, bool kSmag>
@@ -1407,16 +1449,6 @@ __device__ __forceinline__ void block_reduce_add(double (&v)[N], double* out) {
 // lattice, a direction outside 1..18 or an interpolation source outside the
 // lattice skips the link and returns false (the plan's own links are in
 // range by construction).
-// Unfused binary64 forms of r_mul / r_sub / r_fma for the link arithmetic
-// (the binary32 ones already round explicitly); the same bits in every unit,
-// with or without FMA contraction.
-__device__ __forceinline__ float lk_mul(float a, float b) { return r_mul(a, b); }
-__device__ __forceinline__ float lk_sub(float a, float b) { return r_sub(a, b); }
-__device__ __forceinline__ float lk_fma(float a, float b, float c) { return r_fma(a, b, c); }
-__device__ __forceinline__ double lk_mul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double lk_sub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double lk_fma(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
-
 template <class S, bool kChecked = false>
 __device__ __forceinline__ bool add_link3(uint64_t nx, uint64_t plane, uint64_t cells,
                                           const S* __restrict__ f, uint64_t h, int j, double q,

@@ -42,7 +42,7 @@ struct ServeSlot {
     uint32_t ramp_count;    // sampling intervals of the gradual start (0: none)
     const void* ramp;       // inlet velocity of intervals 0 .. ramp_count (3 arithmetic values each;
                             // entry ramp_count is the full inlet velocity)
-    void* inlet;            // the solver's device inlet velocity (3 arithmetic values)
+    void* inlet;            // the solver's device inlet velocity and absorbing targets
     // Evolving.
     uint64_t steps;
     uint64_t window_steps;
@@ -155,6 +155,7 @@ __global__ void serve_period_kernel(ServeSlot* __restrict__ slots, uint32_t n, c
                 to[0] = from[0];
                 to[1] = from[1];
                 to[2] = from[2];
+                for (int i = 0; i < d3::Q; ++i) to[kInletTargets + i] = absorb_target3(i, from);
             }
         }
     }

@@ -271,8 +271,8 @@ orr_status orr_lbm3d_create(const orr_lbm3d_config* config, const uint8_t* solid
             check(cudaMalloc(&hp->hist[0], twice ? 2 * history : history), "outlet buffer");
             hp->hist[1] = twice ? static_cast<char*>(hp->hist[0]) + history : hp->hist[0];
             check(cudaMalloc(&hp->moments, 4 * cells * hp->abytes), "moment buffer");
-            check(cudaMalloc(&hp->small, 256), "small buffer");
-            check(cudaMemsetAsync(hp->small, 0, 256, hp->stream), "small buffer");
+            check(cudaMalloc(&hp->small, kSmallBytes), "small buffer");
+            check(cudaMemsetAsync(hp->small, 0, kSmallBytes, hp->stream), "small buffer");
             check(cudaMallocHost(reinterpret_cast<void**>(&hp->host_small), 256), "pinned buffer");
             check(cudaMalloc(&hp->table, kTableBytes), "lattice table");
         };

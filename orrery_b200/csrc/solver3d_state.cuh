@@ -14,7 +14,8 @@
 //   moments       4 planes (rho or rho - 1, ux, uy, uz) for read-back
 //   history       5 * ny * nz convective-outlet values, twice (a step reads one and
 //                 writes the other; one copy for the zero-gradient outlet)
-//   small         inlet velocity (3), force/moment (6) and mass accumulators,
+//   small         force/moment (6) and mass accumulators, the inlet velocity and its
+//                 absorbing targets,
 //                 the persistent step's status word
 //   table         the lattice-table entry of the persistent step
 // Steps run as CUDA graphs of kGraphSteps steps, one kernel launch each:
@@ -53,6 +54,9 @@ namespace orr {
 constexpr uint32_t kGraphSteps = 16; // even: a graph returns to the buffer it started on
 constexpr uint32_t kDefaultBlock = 128;
 constexpr std::size_t kStatusOffset = 128; // bytes into the small buffer
+constexpr std::size_t kInletOffset = 256;
+constexpr std::size_t kSmallBytes = 512;
+static_assert(kInletOffset + kInletValues * sizeof(double) <= kSmallBytes);
 
 template <class T> T* device_alloc(std::size_t count, const char* what) {
     void* p = nullptr;
@@ -134,7 +138,7 @@ struct orr_lbm3d {
     uint32_t* lcell = nullptr;
     uint32_t* ldir = nullptr;
     double* lq = nullptr;
-    void* small = nullptr;   // inlet (3 x arithmetic) at 0, accumulators at 64
+    void* small = nullptr;   // accumulators at 64, status at kStatusOffset, inlet at kInletOffset
     double* host_small = nullptr; // pinned: inlet staging + results
 
     uint64_t steps = 0;
@@ -146,7 +150,7 @@ struct orr_lbm3d {
         return storage == ORR_STORAGE_F64 ? static_cast<const void*>(&phys64)
                                           : static_cast<const void*>(&phys32);
     }
-    void* inlet_dev() const { return small; }
+    void* inlet_dev() const { return static_cast<char*>(small) + kInletOffset; }
     uint32_t* status() const {
         return reinterpret_cast<uint32_t*>(static_cast<char*>(small) + kStatusOffset);
     }
@@ -163,7 +167,7 @@ struct orr_lbm3d {
         b.wall_count = wall_count;
         b.hist[0] = hist[from];
         b.hist[1] = hist[1 - from];
-        b.inlet = small;
+        b.inlet = inlet_dev();
         return b;
     }
 
@@ -204,14 +208,11 @@ struct orr_lbm3d {
         inlet[2] = v[2];
         check(cudaStreamSynchronize(stream), "inlet upload");
         if (storage == ORR_STORAGE_F64) {
-            std::memcpy(host_small, v, 3 * sizeof(double));
+            fill_inlet(host_small, v);
         } else {
-            float* h = reinterpret_cast<float*>(host_small);
-            h[0] = to_f32(v[0]);
-            h[1] = to_f32(v[1]);
-            h[2] = to_f32(v[2]);
+            fill_inlet(reinterpret_cast<float*>(host_small), v);
         }
-        check(cudaMemcpyAsync(small, host_small, 3 * abytes, cudaMemcpyHostToDevice, stream),
+        check(cudaMemcpyAsync(inlet_dev(), host_small, kInletValues * abytes, cudaMemcpyHostToDevice, stream),
               "inlet upload");
         check(cudaStreamSynchronize(stream), "inlet upload");
     }
