@@ -1213,6 +1213,102 @@ __global__ void __launch_bounds__(256, kStepMinBlocks<S, kWalls>)
     step_node3<S, kSmag, kWalls>(g, p, src, dst, b, x, blockIdx.y, z, 0u);
 }
 
+// Quotients n / d of 32-bit n < 2^31 by multiplication.
+struct FastDiv {
+    uint32_t mul = 0, shift = 0;
+};
+inline FastDiv fast_div(uint32_t d) {
+    // mul = ceil(2^(32 + shift) / d) with 2^shift <= d < 2^(shift + 1): mul d
+    // exceeds 2^(32 + shift) by less than d, so n mul / 2^(32 + shift) is below
+    // n / d + 1 / d while n < 2^31.  A power of two takes half of both.
+    FastDiv f;
+    while ((d >> f.shift) > 1u) ++f.shift;
+    if ((d & (d - 1u)) == 0u) {
+        f.mul = d == 1u ? 0xffffffffu : 1u << 31;
+        f.shift = d == 1u ? 0u : f.shift - 1u;
+    } else {
+        f.mul = static_cast<uint32_t>(((uint64_t{1} << (32 + f.shift)) + d - 1u) / d);
+    }
+    return f;
+}
+__device__ __forceinline__ uint32_t divide(uint32_t n, FastDiv f) { return __umulhi(n, f.mul) >> f.shift; }
+
+// Byte offsets of direction i's pull and store of node 0 from the population
+// buffers.
+struct LinearOffsets3D {
+    uint32_t in[d3::Q], out[d3::Q];
+};
+struct LinearDivs3D {
+    FastDiv nx, ny;
+};
+
+template <class S> __device__ __forceinline__ const S* bytes_from(const S* p, uint32_t n) {
+    return reinterpret_cast<const S*>(reinterpret_cast<const char*>(p) + n);
+}
+template <class S> __device__ __forceinline__ S* bytes_from(S* p, uint32_t n) {
+    return reinterpret_cast<S*>(reinterpret_cast<char*>(p) + n);
+}
+
+// The step of a flat lattice over its nodes in linear order: block k takes
+// the nodes [k B, (k + 1) B) whatever rows they lie in, so no lane is idle at
+// a row's end, every plain pull is issued without a test (each stays inside
+// the buffer for every node: direction i's plane has i planes below it and
+// 18 - i above), and one 32-bit byte offset per access is added to the two
+// buffers' bases (a buffer is below 4 GB).  Bound: instruction issue for the
+// 2-byte storages (82% of the slots), memory for binary32.  Against the row
+// tiles, us per step: binary16 256 x 128 x 128 89.0 -> 79.3, 128 x 110 x 105 40.1
+// -> 34.5, 512 x 256 x 256 640 -> 566, 337 x 193 x 193 268 -> 230; binary32
+// 337 x 193 x 193 334 -> 324, but 256 x 128 x 128 102.9 -> 104.5 (the
+// launcher's rule).  One pair of nodes a thread (96 registers, 25% of the
+// warps) and copy pipelines through shared memory, per block or per warp,
+// measured 82 to 112 us for binary16 256 x 128 x 128.
+template <class S> constexpr int kLinearMinBlocks = sizeof(S) == 2 ? 6 : 5;   // 40 and 48 registers
+
+// (The divisors come last: in front of the tables' pointers they cost the
+// compiler 16 bytes of spills a thread.)
+template <class S, bool kSmag>
+__global__ void __launch_bounds__(256, kLinearMinBlocks<S>)
+    step3d_linear_kernel(Geom3D g, Phys3D<float> p, const S* __restrict__ src, S* __restrict__ dst,
+                         LinearOffsets3D l, StepBuffers3D b, LinearDivs3D d) {
+    using T = Storage<S>;
+    const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h >= static_cast<uint32_t>(g.cells)) {
+        return;
+    }
+    const uint32_t hb = h * static_cast<uint32_t>(sizeof(S));
+    float f[d3::Q];
+#pragma unroll
+    for (int i = 0; i < d3::Q; ++i) {
+        f[i] = T::load(bytes_from(src, hb + l.in[i]));
+    }
+    const uint8_t cls = __ldg(b.cls + h);
+    const uint32_t row = divide(h, d.nx), x = h - row * g.nx;
+    const uint32_t z = divide(row, d.ny), y = row - z * g.ny;
+    if (sizeof(S) == 2 || cls != kBulk || x == 0u || x + 1u == g.nx) {
+        if (cls == kSolid) {
+#pragma unroll
+            for (int i = 0; i < d3::Q; ++i) {
+                T::store(bytes_from(dst, hb + l.out[i]), 0.0f);
+            }
+            return;
+        }
+        const bool interior = (y - 1u < g.ny - 2u) && (z - 1u < g.nz - 2u);
+        flat_fix3<S>(g, p, src, b, f, cls, interior, x, y, z, h, 0u);
+    }
+    float ux, uy, uz;
+    collide3<float, true, kSmag>(f, p, g.forced, ux, uy, uz);
+    if (g.sponge) {
+        const float s = sponge_rate3<float>(g, p, x, y, z);
+        if (s > 0.0f) {
+            absorb3<float>(f, s, static_cast<const float*>(b.inlet));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < d3::Q; ++i) {
+        T::store(bytes_from(dst, hb + l.out[i]), f[i]);
+    }
+}
+
 // Row tiles of neighbouring node pairs, for the 2-byte storage forms of a
 // flat lattice with even nx: thread t of block (k, y, z) takes the nodes
 // x0 = 2 (k B + t) and x0 + 1 of row (y, z).  In an interior row each

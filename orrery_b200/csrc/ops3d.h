@@ -18,8 +18,9 @@ struct StepBuffers3D;
 struct Ops3D {
     // One fused step src -> dst (one launch).  `phys` points at a Phys3D of
     // the storage's arithmetic type; `block` is the block width (threads
-    // along x of a row); npt 2 takes the pair step (two neighbouring nodes
-    // per thread) where pairs_ok allows it, the one-node step otherwise.
+    // along x of a row, or of a linear tile where step_linear says so); npt 2
+    // takes the pair step (two neighbouring nodes per thread) where pairs_ok
+    // allows it, the one-node step otherwise.
     cudaError_t (*step)(const Geom3D& g, const void* phys, const void* src, void* dst,
                         const StepBuffers3D& b, bool smag, uint32_t block, uint32_t npt, cudaStream_t s);
     // Equilibrium initialisation of a population buffer; rho..uz may be
@@ -35,8 +36,10 @@ struct Ops3D {
                          cudaStream_t s);
     cudaError_t (*mass)(const Geom3D& g, const uint8_t* cls, const void* f, double* out,
                         cudaStream_t s);
-    // Registers per thread of the step kernel (for the tuner and the docs).
-    int (*step_registers)(bool smag, uint32_t npt);
+    // Whether the one-node step of lattice g runs in linear order.
+    bool (*step_linear)(const Geom3D& g);
+    // Registers per thread of lattice g's step kernel.
+    int (*step_registers)(const Geom3D& g, bool smag, uint32_t npt);
     // Whether the pair step serves lattice g with blocks of `block` threads
     // (2-byte storage, periodic or free-slip sides and halfway walls, even nx,
     // whole warps up to 128 threads).

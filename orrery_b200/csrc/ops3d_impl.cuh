@@ -33,6 +33,22 @@ template <class S> struct Launch3D {
                 return cudaGetLastError();
             }
         }
+        if constexpr (sizeof(A) == 4) {
+            if (step_linear(g)) {
+                LinearOffsets3D l;
+                for (int i = 0; i < d3::Q; ++i) {
+                    const int64_t to = static_cast<int64_t>(i) * static_cast<int64_t>(g.cells);
+                    const int64_t shift = d3::cx(i) + static_cast<int64_t>(g.nx) * d3::cy(i) +
+                                          static_cast<int64_t>(g.plane) * d3::cz(i);
+                    l.in[i] = static_cast<uint32_t>((to - shift) * static_cast<int64_t>(sizeof(S)));
+                    l.out[i] = static_cast<uint32_t>(to * static_cast<int64_t>(sizeof(S)));
+                }
+                const unsigned blocks = static_cast<unsigned>((g.cells + block - 1) / block);
+                linear_kernel(smag)<<<blocks, block, 0, s>>>(gg, p, in, out, l, b,
+                                                             LinearDivs3D{fast_div(g.nx), fast_div(g.ny)});
+                return cudaGetLastError();
+            }
+        }
         const dim3 grid(gg.tiles_x, g.ny, g.nz);
         const auto launch = [&]<bool K>() {
             if (g.flat) {
@@ -53,6 +69,19 @@ template <class S> struct Launch3D {
             launch.template operator()<false>();
         }
         return cudaGetLastError();
+    }
+
+    // The linear order serves flat lattices whose buffers 32-bit byte offsets
+    // reach.  The 2-byte storages gain from it at every size; binary32, bound
+    // by memory, where rows do not fill their tiles (337 x 193 x 193 334 -> 324
+    // us per step) and not where they do (256 x 128 x 128 102.9 -> 104.5).
+    static bool step_linear(const Geom3D& g) {
+        return sizeof(A) == 4 && g.flat && d3::Q * g.cells * sizeof(S) <= 0xffffffffull &&
+               (sizeof(S) == 2 || g.nx % 64 != 0);
+    }
+
+    static auto linear_kernel(bool smag) {
+        return smag ? &step3d_linear_kernel<S, true> : &step3d_linear_kernel<S, false>;
     }
 
     static cudaError_t init(const Geom3D& g, const uint8_t* cls, const double* rho,
@@ -109,19 +138,27 @@ template <class S> struct Launch3D {
         return sizeof(S) == 2 && g.flat && g.nx % 2 == 0 && block % 32 == 0 && block <= 128;
     }
 
-    static int step_registers(bool smag, uint32_t npt) {
+    static int step_registers(const Geom3D& g, bool smag, uint32_t npt) {
         cudaFuncAttributes a{};
-        cudaError_t e = cudaErrorInvalidValue;
+        const auto registers = [&a](auto kernel) {
+            return cudaFuncGetAttributes(&a, kernel) == cudaSuccess ? a.numRegs : -1;
+        };
         if constexpr (sizeof(S) == 2) {
             if (npt == 2) {
-                e = smag ? cudaFuncGetAttributes(&a, step3d_pair_kernel<S, true>)
-                         : cudaFuncGetAttributes(&a, step3d_pair_kernel<S, false>);
-                return e == cudaSuccess ? a.numRegs : -1;
+                return registers(smag ? &step3d_pair_kernel<S, true> : &step3d_pair_kernel<S, false>);
             }
         }
-        e = smag ? cudaFuncGetAttributes(&a, step3d_kernel<S, true, Walls::Halfway>)
-                 : cudaFuncGetAttributes(&a, step3d_kernel<S, false, Walls::Halfway>);
-        return e == cudaSuccess ? a.numRegs : -1;
+        if constexpr (sizeof(A) == 4) {
+            if (step_linear(g)) {
+                return registers(linear_kernel(smag));
+            }
+        }
+        const auto of = [&]<Walls K>() {
+            return registers(smag ? &step3d_kernel<S, true, K> : &step3d_kernel<S, false, K>);
+        };
+        return g.flat   ? of.template operator()<Walls::Halfway>()
+               : g.open ? of.template operator()<Walls::Interpolated>()
+                        : of.template operator()<Walls::General>();
     }
 
     template <bool kSmag, int B, int NPT, bool kSingle> static constexpr auto staged_kernel() {
@@ -289,7 +326,7 @@ template <class S> struct Launch3D {
 
     static const Ops3D& table() {
         static const Ops3D ops{&step,   &init,   &history,        &moments,          &force,
-                               &mass,   &step_registers, &pairs_ok, &staged, &staged_occupancy,
+                               &mass,   &step_linear, &step_registers, &pairs_ok, &staged, &staged_occupancy,
                                &staged_smem, &staged_registers, &tiled, &tiled_occupancy,
                                &tiled_registers, &force_batch};
         return ops;

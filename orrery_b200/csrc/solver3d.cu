@@ -467,6 +467,10 @@ orr_status orr_lbm3d_create(const orr_lbm3d_config* config, const uint8_t* solid
                                                "and blocks of at most 128 threads"};
             }
             h->row_npt = 2;
+        } else if (o.block_x == 0 && h->ops->step_linear(g)) {
+            // Linear tiles of 256 nodes: binary16 512 x 256 x 256 takes 566 us
+            // per step with 256, 668 with 128; small lattices the same.
+            h->block = 256u;
         }
         initialize_state(h.get(), nullptr, nullptr, nullptr, nullptr);
         // Capture the step graph now, so that no step() call, the first
@@ -761,8 +765,10 @@ orr_status orr_lbm3d_kernel_info(const orr_lbm3d* solver, orr_kernel_info* info)
             k.block = solver->block;
             const uint32_t span = solver->block * solver->row_npt;
             k.nodes_per_thread = solver->row_npt;
-            k.grid = ((solver->g.nx + span - 1) / span) * solver->g.ny * solver->g.nz;
-            k.registers = solver->ops->step_registers(solver->smag, solver->row_npt);
+            k.grid = solver->row_npt == 1 && solver->ops->step_linear(solver->g)
+                         ? static_cast<uint32_t>((solver->g.cells + span - 1) / span)
+                         : ((solver->g.nx + span - 1) / span) * solver->g.ny * solver->g.nz;
+            k.registers = solver->ops->step_registers(solver->g, solver->smag, solver->row_npt);
         }
         *info = k;
         return ORR_OK;
