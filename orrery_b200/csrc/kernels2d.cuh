@@ -22,7 +22,6 @@ namespace orr {
 struct Geom2D {
     uint32_t nx, ny;
     uint64_t cells;
-    uint32_t tiles_x;
     int32_t x_mode, outlet_mode;
     int32_t bottom, top; // ORR_WALL_*
     int32_t forced;
@@ -190,7 +189,7 @@ __device__ __forceinline__ void inlet_west2(A (&f)[d2::Q], A ux, A uy) {
 struct StepBuffers2D {
     const uint8_t* cls;
     const uint32_t* nmask; // per node, bit i: direction i bounces back
-    void* hist;
+    void* hist[2];         // outlet history: a step reads hist[0] and writes hist[1] (StepBuffers3D)
 };
 
 template <class S, int I>
@@ -237,11 +236,10 @@ __device__ __forceinline__ void gather_one2(const Geom2D& g, const Phys2D<typena
             if (g.outlet_mode == ORR_OUTLET_EXTRAPOLATION) {
                 out = up;
             } else {
-                A* hist = static_cast<A*>(b.hist);
                 const uint64_t k = static_cast<uint64_t>(d2::outlet_slot(I)) * g.ny + static_cast<uint64_t>(y);
                 const A u = p.outlet_speed;
-                const A v = (hist[k] + u * up) / (A(1) + u);
-                hist[k] = v;
+                const A v = (static_cast<const A*>(b.hist[0])[k] + u * up) / (A(1) + u);
+                static_cast<A*>(b.hist[1])[k] = v;
                 out = v;
             }
             return;
@@ -267,68 +265,103 @@ __device__ __forceinline__ void gather_all2(const Geom2D& g, const Phys2D<typena
     }
 }
 
-// One fused step src -> dst: one thread per node, one block per row tile,
-// all rows; solid lanes store their rest populations, bulk lanes (interior
-// rows, x-edges shifted) pull plainly, face and boundary lanes take the
-// general gather (see step3d_kernel for the reasons).
-template <class S, bool kSmag>
-__global__ void __launch_bounds__(256) step2d_kernel(Geom2D g, Phys2D<typename Storage<S>::A> p,
-                                                     const S* __restrict__ src, S* __restrict__ dst,
-                                                     StepBuffers2D b) {
+// Byte offsets of direction i's pull and store of node 0, and of the last
+// value of a buffer, in 32 bits or (buffers of 4 GB and more) 64.
+template <class O> struct LinearOffsets2D {
+    O in[d2::Q], out[d2::Q], last;
+};
+
+// One fused step src -> dst over the nodes in linear order (see
+// step3d_linear_kernel): the 9 plain pulls are issued untested together with
+// the class byte (direction 8 of the last row would read past the buffer and
+// is held at its last value), then the few lanes that are not plain bulk
+// nodes take their rules: solid nodes store their rest populations, boundary
+// nodes of inner rows replace their solid-source pulls by f*_opp, the others
+// take the general gather.  Bound: memory, and launch latency for small
+// lattices.  When a lane waited for its class before its pulls, with 64-bit
+// addresses and the history in place -> now, us per step: 2048 x 1024 binary32
+// 34.9 -> 27.4 (convective, BGK; floor 23.1) and 34.9 -> 28.4 (zero gradient,
+// closure), binary64 58.0 -> 54.1 and 71.5 -> 61.6; 400 x 160 binary32 4.74 ->
+// 4.10 and 3.72 -> 3.59.
+//
+// 40 registers for binary32 arithmetic and 64 for binary64: 2048 x 1024
+// binary32 takes 27.1 us with 40, 28.8 with 48 and 27.2 with 32 (spills);
+// binary64 with the closure 62.0 with 64, 64.7 with 78 and 80.4 with 48.
+template <class S> constexpr int kStep2dMinBlocks = sizeof(typename Storage<S>::A) == 8 ? 4 : 6;
+
+template <class S, bool kSmag, class O>
+__global__ void __launch_bounds__(256, kStep2dMinBlocks<S>)
+    step2d_kernel(Geom2D g, Phys2D<typename Storage<S>::A> p, const S* __restrict__ src, S* __restrict__ dst,
+                  LinearOffsets2D<O> l, StepBuffers2D b, FastDiv by_nx) {
     using A = typename Storage<S>::A;
     using T = Storage<S>;
-    const uint32_t y = blockIdx.x / g.tiles_x;
-    const uint32_t x = (blockIdx.x - y * g.tiles_x) * blockDim.x + threadIdx.x;
-    if (x >= g.nx) {
+    const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h >= static_cast<uint32_t>(g.cells)) {
         return;
     }
-    const uint64_t here = x + static_cast<uint64_t>(g.nx) * y;
-    const uint8_t cls = b.cls[here];
-    if (cls == kSolid) {
-#pragma unroll
-        for (int i = 0; i < d2::Q; ++i) {
-            T::store(dst + static_cast<uint64_t>(i) * g.cells + here, T::kShifted ? A(0) : A(d2::w(i)));
-        }
-        return;
-    }
+    const uint32_t y = divide(h, by_nx), x = h - y * g.nx;
+    const bool xlo = x == 0u, xhi = x + 1u == g.nx, periodic = g.x_mode == ORR_X_PERIODIC;
+    const O hb = static_cast<O>(h) * static_cast<O>(sizeof(S));
+    // The x-edge lanes read their x sources from the wrapped column (periodic)
+    // or the outlet's own (zero gradient); an inlet's unknowns are not used.
+    const O east = xlo && periodic ? hb + static_cast<O>(g.nx * sizeof(S)) : hb;
+    const O west = xhi ? hb - static_cast<O>((periodic ? g.nx : 1u) * sizeof(S)) : hb;
     A f[d2::Q];
-    if (cls == kBulk) {
-        const int64_t nx = g.nx;
-        const bool xlo = x == 0u, xhi = x + 1u == g.nx;
-        const int64_t shift_lo = g.x_mode == ORR_X_PERIODIC ? nx : 0;
-        const int64_t shift_hi = g.x_mode == ORR_X_PERIODIC ? -nx : -1;
 #pragma unroll
-        for (int i = 0; i < d2::Q; ++i) {
-            int64_t source = static_cast<int64_t>(here) - (d2::cx(i) + nx * d2::cy(i));
-            if (d2::cx(i) > 0 && xlo) source += shift_lo;
-            if (d2::cx(i) < 0 && xhi) source += shift_hi;
-            f[i] = T::load(src + static_cast<uint64_t>(i) * g.cells + static_cast<uint64_t>(source));
-        }
-        if (xhi && g.x_mode == ORR_X_INFLOW_OUTFLOW && g.outlet_mode == ORR_OUTLET_CONVECTIVE) {
-            A* hist = static_cast<A*>(b.hist);
-            const A u = p.outlet_speed;
+    for (int i = 0; i < d2::Q; ++i) {
+        const O at = (d2::cx(i) > 0 ? east : d2::cx(i) < 0 ? west : hb) + l.in[i];
+        f[i] = T::load(bytes_from(src, i == 8 ? min(at, l.last) : at));
+    }
+    const uint8_t cls = __ldg(b.cls + h);
+    if (cls != kBulk || xlo || xhi) {
+        if (cls == kSolid) {
 #pragma unroll
             for (int i = 0; i < d2::Q; ++i) {
-                if (d2::cx(i) < 0) {
-                    const uint64_t k = static_cast<uint64_t>(d2::outlet_slot(i)) * g.ny + y;
-                    const A v = (hist[k] + u * f[i]) / (A(1) + u);
-                    hist[k] = v;
-                    f[i] = v;
+                T::store(bytes_from(dst, hb + l.out[i]), T::kShifted ? A(0) : A(d2::w(i)));
+            }
+            return;
+        }
+        const uint64_t here = h;
+        if (cls == kBulk) {
+            if (xhi && !periodic && g.outlet_mode == ORR_OUTLET_CONVECTIVE) {
+                const A u = p.outlet_speed;
+                A old[d2::kOutletSlots];
+#pragma unroll
+                for (int k = 0; k < d2::kOutletSlots; ++k) {
+                    old[k] = static_cast<const A*>(b.hist[0])[static_cast<uint64_t>(k) * g.ny + y];
+                }
+#pragma unroll
+                for (int i = 0; i < d2::Q; ++i) {
+                    if (d2::cx(i) < 0) {
+                        const A v = (old[d2::outlet_slot(i)] + u * f[i]) / (A(1) + u);
+                        static_cast<A*>(b.hist[1])[static_cast<uint64_t>(d2::outlet_slot(i)) * g.ny + y] = v;
+                        f[i] = v;
+                    }
                 }
             }
+        } else {
+            const uint32_t mask = cls == kBoundary ? b.nmask[here] : 0u;
+            if (cls == kBoundary && y - 1u < g.ny - 2u && !xlo && !xhi) {
+#pragma unroll
+                for (int i = 0; i < d2::Q; ++i) {
+                    if ((mask >> i) & 1u) {
+                        f[i] = T::load(src + static_cast<uint64_t>(d2::opposite(i)) * g.cells + here);
+                    }
+                }
+            } else {
+                A wall_rho = A(-1);
+                gather_all2<S, 0>(g, p, src, b, mask, static_cast<int>(x), static_cast<int>(y), here, wall_rho, f);
+            }
         }
-    } else {
-        const uint32_t mask = cls == kBoundary ? b.nmask[here] : 0u;
-        A wall_rho = A(-1);
-        gather_all2<S, 0>(g, p, src, b, mask, static_cast<int>(x), static_cast<int>(y), here,
-                          wall_rho, f);
-    }
-    if (g.x_mode == ORR_X_INFLOW_OUTFLOW && x == 0u) {
-        inlet_west2<A, T::kShifted>(f, p.inlet_ux, p.inlet_uy);
+        if (g.x_mode == ORR_X_INFLOW_OUTFLOW && xlo) {
+            inlet_west2<A, T::kShifted>(f, p.inlet_ux, p.inlet_uy);
+        }
     }
     collide2<A, T::kShifted, kSmag>(f, p, g.forced);
 #pragma unroll
-    for (int i = 0; i < d2::Q; ++i) T::store(dst + static_cast<uint64_t>(i) * g.cells + here, f[i]);
+    for (int i = 0; i < d2::Q; ++i) {
+        T::store(bytes_from(dst, hb + l.out[i]), f[i]);
+    }
 }
 
 // Equilibrium initialisation (initial_populations, lbm2d_common.cpp:178-193).

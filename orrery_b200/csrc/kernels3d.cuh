@@ -1242,10 +1242,10 @@ struct LinearDivs3D {
     FastDiv nx, ny;
 };
 
-template <class S> __device__ __forceinline__ const S* bytes_from(const S* p, uint32_t n) {
+template <class S, class O> __device__ __forceinline__ const S* bytes_from(const S* p, O n) {
     return reinterpret_cast<const S*>(reinterpret_cast<const char*>(p) + n);
 }
-template <class S> __device__ __forceinline__ S* bytes_from(S* p, uint32_t n) {
+template <class S, class O> __device__ __forceinline__ S* bytes_from(S* p, O n) {
     return reinterpret_cast<S*>(reinterpret_cast<char*>(p) + n);
 }
 

@@ -12,16 +12,27 @@ template <class S> struct Launch2D {
     using A = typename Storage<S>::A;
     static cudaError_t step(const Geom2D& g, const void* phys, const void* src, void* dst,
                             const StepBuffers2D& b, bool smag, uint32_t block, cudaStream_t s) {
-        Geom2D gg = g;
-        gg.tiles_x = (g.nx + block - 1) / block;
-        const unsigned blocks = g.ny * gg.tiles_x;
+        const unsigned blocks = static_cast<unsigned>((g.cells + block - 1) / block);
         const auto& p = *static_cast<const Phys2D<A>*>(phys);
-        if (smag) {
-            step2d_kernel<S, true><<<blocks, block, 0, s>>>(gg, p, static_cast<const S*>(src),
-                                                            static_cast<S*>(dst), b);
+        const auto launch = [&]<class O>() {
+            LinearOffsets2D<O> l;
+            for (int i = 0; i < d2::Q; ++i) {
+                const int64_t to = static_cast<int64_t>(i) * static_cast<int64_t>(g.cells);
+                const int64_t shift = d2::cx(i) + static_cast<int64_t>(g.nx) * d2::cy(i);
+                l.in[i] = static_cast<O>((to - shift) * static_cast<int64_t>(sizeof(S)));
+                l.out[i] = static_cast<O>(to * static_cast<int64_t>(sizeof(S)));
+            }
+            l.last = static_cast<O>((d2::Q * g.cells - 1) * sizeof(S));
+            const auto kernel = smag ? &step2d_kernel<S, true, O> : &step2d_kernel<S, false, O>;
+            kernel<<<blocks, block, 0, s>>>(g, p, static_cast<const S*>(src), static_cast<S*>(dst), l, b,
+                                            fast_div(g.nx));
+        };
+        // Past the buffer's end by at most a row before it is held: the sums
+        // must not wrap.
+        if ((d2::Q * g.cells + g.nx) * sizeof(S) <= 0xffffffffull) {
+            launch.template operator()<uint32_t>();
         } else {
-            step2d_kernel<S, false><<<blocks, block, 0, s>>>(gg, p, static_cast<const S*>(src),
-                                                             static_cast<S*>(dst), b);
+            launch.template operator()<uint64_t>();
         }
         return cudaGetLastError();
     }

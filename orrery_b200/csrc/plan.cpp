@@ -738,7 +738,8 @@ std::optional<std::size_t> memory2d(const orr_lbm2d_config& c, std::size_t links
     }
     const std::size_t cells = c.nx * c.ny;
     const std::size_t s = storage_bytes(storage), a = arithmetic_bytes(storage);
-    return cells * (d2::Q * s * 2 + 1 + 3 * a) + c.ny * d2::kOutletSlots * a +
+    return cells * (d2::Q * s * 2 + 1 + 3 * a) +
+           c.ny * d2::kOutletSlots * a * (c.outlet == ORR_OUTLET_CONVECTIVE ? 2 : 1) +
            cells * 4 + links * 8 + 256;
 }
 
