@@ -15,6 +15,7 @@
 
 #include "common.h"
 #include "trace.h"
+#include "host_copy.h"
 #include "kernels2d.cuh"
 #include "lattice.h"
 #include "ops2d.h"
@@ -173,11 +174,12 @@ void initialize2(orr_lbm2d* h, const double* rho, const double* ux, const double
     if (rho != nullptr) {
         double* base = static_cast<double*>(h->f[1]);
         const double* src[3] = {rho, ux, uy};
+        orr::HostSpan spans[3];
         for (int k = 0; k < 3; ++k) {
             staged[k] = base + static_cast<std::size_t>(k) * cells;
-            check(cudaMemcpyAsync(staged[k], src[k], cells * 8, cudaMemcpyHostToDevice, h->stream),
-                  "initial state upload");
+            spans[k] = {const_cast<double*>(src[k]), staged[k], cells * 8};
         }
+        orr::copy_to_device(spans, 3, h->stream, h->device);
     }
     const bool inflow = c.x_boundary == ORR_X_INFLOW_OUTFLOW;
     check(h->ops->init(h->g, h->cls, staged[0], staged[1], staged[2], inflow ? c.inlet_ux : 0.0,
@@ -375,24 +377,18 @@ orr_status orr_lbm2d_macroscopic(orr_lbm2d* solver, double* rho, double* ux, dou
         check(h->ops->moments(h->g, h->phys(), h->cls, h->f[h->cur], h->moments, h->stream), "moments kernel");
         ++h->launches;
         double* outs[3] = {rho, ux, uy};
+        // As the D3Q19 fields: binary32 planes cross the bus as they are and
+        // the host threads widen them (rho with 1 added back).
         const bool shifted = h->storage != ORR_STORAGE_F64;
-        std::vector<float> tmp(shifted ? cells : 0);
+        orr::HostSpan spans[3];
+        int count = 0;
         for (int k = 0; k < 3; ++k) {
-            if (outs[k] == nullptr) continue;
-            const char* plane = static_cast<const char*>(h->moments) + k * cells * h->abytes;
-            if (shifted) {
-                check(cudaMemcpyAsync(tmp.data(), plane, cells * 4, cudaMemcpyDeviceToHost, h->stream),
-                      "moment read-back");
-                check(cudaStreamSynchronize(h->stream), "moment read-back");
-                for (std::size_t c = 0; c < cells; ++c) {
-                    outs[k][c] = static_cast<double>(tmp[c]) + (k == 0 ? 1.0 : 0.0);
-                }
-            } else {
-                check(cudaMemcpyAsync(outs[k], plane, cells * 8, cudaMemcpyDeviceToHost, h->stream),
-                      "moment read-back");
-                check(cudaStreamSynchronize(h->stream), "moment read-back");
+            if (outs[k] != nullptr) {
+                spans[count++] = {outs[k], static_cast<char*>(h->moments) + k * cells * h->abytes,
+                                  cells * h->abytes, shifted, shifted && k == 0 ? 1.0 : 0.0};
             }
         }
+        orr::copy_to_host(spans, count, h->stream, h->device);
         return ORR_OK;
     });
 }
@@ -405,8 +401,16 @@ orr_status orr_lbm2d_populations(orr_lbm2d* solver, double* f) {
         }
         const std::size_t cells = h->plan.cells, n = d2::Q * cells;
         if (h->storage == ORR_STORAGE_F64) {
-            check(cudaMemcpyAsync(f, h->f[h->cur], n * 8, cudaMemcpyDeviceToHost, h->stream), "population read-back");
-            check(cudaStreamSynchronize(h->stream), "population read-back");
+            const orr::HostSpan all{f, h->f[h->cur], n * 8};
+            orr::copy_to_host(&all, 1, h->stream, h->device);
+            return ORR_OK;
+        }
+        if (h->storage == ORR_STORAGE_F32) {
+            orr::HostSpan spans[d2::Q];
+            for (int i = 0; i < d2::Q; ++i) {
+                spans[i] = {f + i * cells, static_cast<float*>(h->f[h->cur]) + i * cells, cells * 4, true, d2::w(i)};
+            }
+            orr::copy_to_host(spans, d2::Q, h->stream, h->device);
             return ORR_OK;
         }
         std::vector<unsigned char> raw(n * h->sbytes);
@@ -418,11 +422,7 @@ orr_status orr_lbm2d_populations(orr_lbm2d* solver, double* f) {
             for (std::size_t c = 0; c < cells; ++c) {
                 const std::size_t k = static_cast<std::size_t>(i) * cells + c;
                 double v;
-                if (h->storage == ORR_STORAGE_F32) {
-                    float x;
-                    std::memcpy(&x, raw.data() + 4 * k, 4);
-                    v = x;
-                } else if (h->storage == ORR_STORAGE_F16) {
+                if (h->storage == ORR_STORAGE_F16) {
                     __half x;
                     std::memcpy(&x, raw.data() + 2 * k, 2);
                     v = static_cast<double>(__half2float(x));
