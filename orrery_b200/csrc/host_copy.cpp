@@ -28,7 +28,7 @@ namespace {
 constexpr std::size_t kChunk = std::size_t(4) << 20;
 constexpr int kSlots = 8;
 constexpr int kMaxWorkers = 16;
-constexpr std::size_t kBytesPerWorker = std::size_t(2) << 20;
+constexpr std::size_t kAloneBytes = std::size_t(4) << 20;
 
 // One staged copy at a time in the process: the ring is shared.  It is
 // allocated on first use (portable, so every device's DMA can use it) and
@@ -138,15 +138,14 @@ void staged(bool upload, const std::vector<Chunk>& chunks, cudaStream_t stream, 
     unsigned char* slots = ring();
     Events ev;
     const std::size_t n = chunks.size();
-    // A thread per 2 MiB of host memory, up to the copy's full count: a small
-    // widening read-back (a 64 x 32 x 32 lattice's fields: 2 MiB) takes less
-    // time on this thread than sixteen threads take to start.
+    // A small widening read-back (a 64 x 32 x 32 lattice's fields: 2 MiB)
+    // takes less time on one thread than sixteen take to start.  A larger copy
+    // keeps them all: its pages fault in faster on more threads.
     std::size_t host_bytes = 0;
     for (const Chunk& c : chunks) {
         host_bytes += c.widen ? 2 * c.len : c.len;
     }
-    const int nworkers = static_cast<int>(std::clamp<std::size_t>(
-        host_bytes / kBytesPerWorker, 1, static_cast<std::size_t>(worker_count(upload))));
+    const int nworkers = host_bytes <= kAloneBytes ? 1 : worker_count(upload);
     Progress pr;
     pr.filled.assign(n, 0);
     const auto slot = [&](std::size_t j) { return slots + (j % kSlots) * kChunk; };
