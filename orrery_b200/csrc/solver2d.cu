@@ -172,6 +172,12 @@ void initialize2(orr_lbm2d* h, const double* rho, const double* ux, const double
     const std::size_t cells = h->plan.cells;
     double* staged[3] = {nullptr, nullptr, nullptr};
     if (rho != nullptr) {
+        // The fields are staged in the second population buffer: three
+        // binary64 planes, 24 bytes per node, where the 2-byte storages have 18.
+        // Refused before the copy: a chunk of it could start in the next allocation.
+        if (3 * sizeof(double) > d2::Q * h->sbytes) {
+            throw CudaError{cudaErrorInvalidValue, "initial state upload"};
+        }
         double* base = static_cast<double*>(h->f[1]);
         const double* src[3] = {rho, ux, uy};
         orr::HostSpan spans[3];

@@ -71,3 +71,23 @@ def test_64_bit_offsets_keep_a_uniform_stream():
     assert np.max(np.abs(m.density - 1.0)) < 1e-13
     assert np.max(np.abs(m.velocity_x - 0.05)) < 1e-13
     assert np.max(np.abs(m.velocity_y)) < 1e-13
+
+
+# Initial fields are staged in a population buffer, which the 2-byte storages
+# have no room for: refused before the copy, direct or through the ring, and
+# the solver keeps its state.
+@pytest.mark.parametrize("storage", ["f16", "bf16"])
+@pytest.mark.parametrize("size", [(64, 32), (2048, 1024)])
+def test_two_byte_storages_refuse_initial_fields(size, storage):
+    nx, ny = size
+    c = Lbm2DConfig(nx=nx, ny=ny, tau=0.6, x_boundary=XBoundary.inflow_outflow, outlet=Outlet.convective,
+                    bottom=wall(WallKind.slip), top=wall(WallKind.slip), inlet_ux=0.05)
+    s = S.make_gpu_solver(c, M.fluid_mask(nx, ny), storage=storage)
+    s.step(3)
+    before = s.populations()
+    n = nx * ny
+    with pytest.raises(S.LbmError):
+        s.initialize(np.ones(n), np.full(n, 0.05), np.zeros(n))
+    assert np.array_equal(s.populations(), before)
+    s.step(17)
+    assert np.all(np.isfinite(s.populations()))
