@@ -453,8 +453,10 @@ __global__ void moments2d_kernel(Geom2D g, Phys2D<typename Storage<S>::A> p, con
 // Force2D over the links: 2 c_o f*_o at the halfway wall point, binary64
 // (CpuLbm2D::force, lbm2d_cpu.cpp:265-272; add_link_force, lbm2d.h:145-155).
 template <class S>
-__global__ void force2d_kernel(Geom2D g, const S* __restrict__ f, const uint32_t* __restrict__ lcell,
-                               const uint32_t* __restrict__ ldir, uint64_t links, double* __restrict__ out) {
+__global__ void __launch_bounds__(kForceThreads) force2d_kernel(Geom2D g, const S* __restrict__ f,
+                                                                const uint32_t* __restrict__ lcell,
+                                                                const uint32_t* __restrict__ ldir, uint64_t links,
+                                                                ForceScratch* scratch, double* result) {
     using T = Storage<S>;
     double acc[3] = {0, 0, 0};
     for (uint64_t k = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < links;
@@ -475,7 +477,7 @@ __global__ void force2d_kernel(Geom2D g, const S* __restrict__ f, const uint32_t
         acc[1] += fy;
         acc[2] += rx * fy - ry * fx;
     }
-    block_reduce_add<3>(acc, out);
+    finish_force<3>(acc, scratch, result, nullptr);
 }
 
 template <class S>

@@ -1608,19 +1608,97 @@ __device__ __forceinline__ bool add_link3(uint64_t nx, uint64_t plane, uint64_t 
     return true;
 }
 
+// Blocks of the solvers' force kernels, at most: two per SM.
+constexpr uint32_t kForceBlocks = 296;
+constexpr uint32_t kForceThreads = 256;
+
+// Sum of N doubles over the block in a fixed order; valid in thread 0.
+template <int N> __device__ __forceinline__ void block_sum_fixed(double (&v)[N]) {
+    __shared__ double part[N][kForceThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) part[k][warp] = v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            double t = 0.0;
+            for (int w = 0; w < static_cast<int>(kForceThreads / 32); ++w) t += part[k][w];
+            v[k] = t;
+        }
+    }
+}
+
+// Scratch of a solver's force kernel: the blocks' sums and the count of
+// blocks done (zero between launches).
+struct ForceScratch {
+    double partial[kForceBlocks][6];
+    uint32_t done;
+};
+
+// End of a force kernel: the block's sums go to the scratch; the last block
+// to arrive adds all of them in block order, resets the count and writes the
+// totals, with the word at `status` (when given), to `result` in pinned host
+// memory.  One launch and no copy: a call on the 64 x 32 x 32 lattice took
+// 32.7 us with a clear, an atomic sum and a read-back, 29.3 us now, most of
+// it the caller's synchronisation.
+template <int N>
+__device__ __forceinline__ void finish_force(double (&acc)[N], ForceScratch* scratch, double* result,
+                                             const uint32_t* status) {
+    __shared__ bool last;
+    block_sum_fixed(acc);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) scratch->partial[blockIdx.x][k] = acc[k];
+        __threadfence();
+        last = atomicAdd(&scratch->done, 1u) + 1u == gridDim.x;
+    }
+    __syncthreads();
+    if (!last) {
+        return;
+    }
+    __threadfence();
+#pragma unroll
+    for (int k = 0; k < N; ++k) acc[k] = 0.0;
+    for (uint32_t b = threadIdx.x; b < gridDim.x; b += kForceThreads) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) acc[k] += __ldcg(&scratch->partial[b][k]);
+    }
+    __syncthreads();
+    block_sum_fixed(acc);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) result[k] = acc[k];
+        if (status != nullptr) {
+            *reinterpret_cast<uint32_t*>(result + N) = *status;
+        }
+        scratch->done = 0u;
+        __threadfence_system();
+    }
+}
+
 // Momentum exchange over the boundary links, summed in binary64 (one thread
-// per link, add_link3; warp shuffles, a block reduction and one atomic per
-// value and block).
+// per link, add_link3).
 template <class S>
-__global__ void force3d_kernel(Geom3D g, const S* __restrict__ f, const uint32_t* __restrict__ lcell,
-                               const uint32_t* __restrict__ ldir, const double* __restrict__ lq,
-                               uint64_t links, double* __restrict__ out) {
+__global__ void __launch_bounds__(kForceThreads) force3d_kernel(Geom3D g, const S* __restrict__ f,
+                                                                const uint32_t* __restrict__ lcell,
+                                                                const uint32_t* __restrict__ ldir,
+                                                                const double* __restrict__ lq, uint64_t links,
+                                                                ForceScratch* scratch, double* result,
+                                                                const uint32_t* status) {
     double acc[6] = {0, 0, 0, 0, 0, 0};
     for (uint64_t k = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < links;
          k += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         add_link3<S>(g.nx, g.plane, g.cells, f, lcell[k], static_cast<int>(ldir[k]), lq[k], acc);
     }
-    block_reduce_add<6>(acc, out);
+    finish_force<6>(acc, scratch, result, status);
 }
 
 // ------------------------------------------------------ batched forces --
@@ -1636,32 +1714,7 @@ struct ForceJob {
     uint64_t nx, plane, cells;
 };
 
-constexpr uint32_t kForceThreads = 256;
 constexpr uint64_t kForceChunk = 2048; // links per block of pass 1
-
-// Sum of six doubles over the block in a fixed order; valid in thread 0.
-__device__ __forceinline__ void block_sum6_fixed(double (&v)[6]) {
-    __shared__ double part[6][kForceThreads / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) part[k][warp] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            double t = 0.0;
-            for (int w = 0; w < static_cast<int>(kForceThreads / 32); ++w) t += part[k][w];
-            v[k] = t;
-        }
-    }
-}
 
 // Pass 1 of the batched force: block b sums global chunk b (kForceChunk
 // links of one lattice) into partial[6 b .. 6 b + 5].
@@ -1686,7 +1739,7 @@ __global__ void __launch_bounds__(kForceThreads) force_batch_partials(const Forc
     for (uint64_t k = begin + threadIdx.x; k < end; k += kForceThreads) {
         add_link3<S>(J.nx, J.plane, J.cells, f, J.lcell[k], static_cast<int>(J.ldir[k]), J.lq[k], acc);
     }
-    block_sum6_fixed(acc);
+    block_sum_fixed(acc);
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int v = 0; v < 6; ++v) partial[chunk * 6 + v] = acc[v];
@@ -1707,7 +1760,7 @@ __global__ void __launch_bounds__(kForceThreads) force_batch_totals(const ForceJ
 #pragma unroll
         for (int v = 0; v < 6; ++v) acc[v] += partial[(J.chunk_begin + c) * 6 + v];
     }
-    block_sum6_fixed(acc);
+    block_sum_fixed(acc);
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int v = 0; v < 6; ++v) {

@@ -10,6 +10,7 @@ namespace orr {
 
 struct Geom2D;
 struct StepBuffers2D;
+struct ForceScratch;
 
 struct Ops2D {
     // One fused step src -> dst (one launch over all rows).
@@ -21,7 +22,8 @@ struct Ops2D {
     cudaError_t (*moments)(const Geom2D& g, const void* phys, const uint8_t* cls, const void* f,
                            void* m, cudaStream_t s);
     cudaError_t (*force)(const Geom2D& g, const void* f, const uint32_t* lcell,
-                         const uint32_t* ldir, uint64_t links, double* out, cudaStream_t s);
+                         const uint32_t* ldir, uint64_t links, ForceScratch* scratch, double* result,
+                         cudaStream_t s); // result: 3 values in pinned host memory
     cudaError_t (*mass)(const Geom2D& g, const uint8_t* cls, const void* f, double* out,
                         cudaStream_t s);
 };

@@ -60,13 +60,12 @@ template <class S> struct Launch2D {
     }
 
     static cudaError_t force(const Geom2D& g, const void* f, const uint32_t* lcell,
-                             const uint32_t* ldir, uint64_t links, double* out, cudaStream_t s) {
-        cudaError_t e = cudaMemsetAsync(out, 0, 3 * sizeof(double), s);
-        if (e != cudaSuccess || links == 0) {
-            return e;
-        }
-        const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((links + 255) / 256, 1184));
-        force2d_kernel<S><<<blocks, 256, 0, s>>>(g, static_cast<const S*>(f), lcell, ldir, links, out);
+                             const uint32_t* ldir, uint64_t links, ForceScratch* scratch, double* result,
+                             cudaStream_t s) {
+        const auto blocks = static_cast<unsigned>(
+            std::clamp<uint64_t>((links + kForceThreads - 1) / kForceThreads, 1, kForceBlocks));
+        force2d_kernel<S><<<blocks, kForceThreads, 0, s>>>(g, static_cast<const S*>(f), lcell, ldir, links, scratch,
+                                                           result);
         return cudaGetLastError();
     }
 

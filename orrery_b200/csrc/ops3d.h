@@ -14,6 +14,7 @@ namespace orr {
 
 struct Geom3D;
 struct StepBuffers3D;
+struct ForceScratch;
 
 struct Ops3D {
     // One fused step src -> dst (one launch).  `phys` points at a Phys3D of
@@ -31,9 +32,11 @@ struct Ops3D {
     cudaError_t (*history)(const Geom3D& g, const void* f, void* hist, cudaStream_t s);
     cudaError_t (*moments)(const Geom3D& g, const void* phys, const uint8_t* cls, const void* f,
                            void* m, cudaStream_t s);
+    // Force and moment into `result`, 6 values in pinned host memory, and the
+    // word at `status` (may be null) after them; `scratch` is the solver's.
     cudaError_t (*force)(const Geom3D& g, const void* f, const uint32_t* lcell,
-                         const uint32_t* ldir, const double* lq, uint64_t links, double* out,
-                         cudaStream_t s);
+                         const uint32_t* ldir, const double* lq, uint64_t links, ForceScratch* scratch,
+                         double* result, const uint32_t* status, cudaStream_t s);
     cudaError_t (*mass)(const Geom3D& g, const uint8_t* cls, const void* f, double* out,
                         cudaStream_t s);
     // Whether the one-node step of lattice g runs in linear order.

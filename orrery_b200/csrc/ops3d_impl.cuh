@@ -109,15 +109,12 @@ template <class S> struct Launch3D {
     }
 
     static cudaError_t force(const Geom3D& g, const void* f, const uint32_t* lcell,
-                             const uint32_t* ldir, const double* lq, uint64_t links, double* out,
-                             cudaStream_t s) {
-        cudaError_t e = cudaMemsetAsync(out, 0, 6 * sizeof(double), s);
-        if (e != cudaSuccess || links == 0) {
-            return e;
-        }
-        const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((links + 255) / 256, 1184));
-        force3d_kernel<S><<<blocks, 256, 0, s>>>(g, static_cast<const S*>(f), lcell, ldir, lq,
-                                                 links, out);
+                             const uint32_t* ldir, const double* lq, uint64_t links, ForceScratch* scratch,
+                             double* result, const uint32_t* status, cudaStream_t s) {
+        const auto blocks = static_cast<unsigned>(
+            std::clamp<uint64_t>((links + kForceThreads - 1) / kForceThreads, 1, kForceBlocks));
+        force3d_kernel<S><<<blocks, kForceThreads, 0, s>>>(g, static_cast<const S*>(f), lcell, ldir, lq, links,
+                                                           scratch, result, status);
         return cudaGetLastError();
     }
 

@@ -27,6 +27,8 @@ using namespace orr;
 
 constexpr uint32_t kGraphSteps2 = 16;
 constexpr uint32_t kDefaultBlock2 = 128;
+constexpr std::size_t kSmallBytes2 = 16384;
+static_assert(8 * sizeof(double) + sizeof(orr::ForceScratch) <= kSmallBytes2);
 
 const Ops2D& ops2_for(int32_t storage) {
     switch (storage) {
@@ -64,7 +66,7 @@ struct orr_lbm2d {
     void* moments = nullptr;
     uint32_t* lcell = nullptr;
     uint32_t* ldir = nullptr;
-    double* acc = nullptr;
+    double* acc = nullptr; // mass sum at 4; the force kernel's scratch from 8
     double* host_acc = nullptr;
     uint64_t steps = 0, launches = 0;
     std::string error;
@@ -301,7 +303,8 @@ orr_status orr_lbm2d_create(const orr_lbm2d_config* config, const uint8_t* solid
               "link buffer");
         check(cudaMalloc(reinterpret_cast<void**>(&h->ldir), std::max<std::size_t>(p.link_cell.size(), 1) * 4),
               "link buffer");
-        check(cudaMalloc(reinterpret_cast<void**>(&h->acc), 8 * sizeof(double)), "accumulator");
+        check(cudaMalloc(reinterpret_cast<void**>(&h->acc), kSmallBytes2), "accumulator");
+        check(cudaMemsetAsync(h->acc, 0, kSmallBytes2, h->stream), "accumulator");
         check(cudaMallocHost(reinterpret_cast<void**>(&h->host_acc), 8 * sizeof(double)), "pinned buffer");
         cudaStream_t s = h->stream;
         check(cudaMemcpyAsync(h->cls, p.cls.data(), cells, cudaMemcpyHostToDevice, s), "class upload");
@@ -366,10 +369,15 @@ orr_status orr_lbm2d_force(orr_lbm2d* solver, double force_moment[3]) {
             throw Refusal{ORR_ERR_INVALID, "null output"};
         }
         const std::size_t links = h->plan.link_cell.size();
-        check(h->ops->force(h->g, h->f[h->cur], h->lcell, h->ldir, links, h->acc, h->stream), "force kernel");
-        if (links > 0) ++h->launches;
-        check(cudaMemcpyAsync(h->host_acc, h->acc, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream),
-              "force read-back");
+        if (links == 0) {
+            check(cudaStreamSynchronize(h->stream), "force read-back");
+            std::fill_n(force_moment, 3, 0.0);
+            return ORR_OK;
+        }
+        check(h->ops->force(h->g, h->f[h->cur], h->lcell, h->ldir, links,
+                            reinterpret_cast<orr::ForceScratch*>(h->acc + 8), h->host_acc, h->stream),
+              "force kernel");
+        ++h->launches;
         check(cudaStreamSynchronize(h->stream), "force read-back");
         std::memcpy(force_moment, h->host_acc, 3 * sizeof(double));
         return ORR_OK;

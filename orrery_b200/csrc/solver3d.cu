@@ -273,7 +273,7 @@ orr_status orr_lbm3d_create(const orr_lbm3d_config* config, const uint8_t* solid
             check(cudaMalloc(&hp->moments, 4 * cells * hp->abytes), "moment buffer");
             check(cudaMalloc(&hp->small, kSmallBytes), "small buffer");
             check(cudaMemsetAsync(hp->small, 0, kSmallBytes, hp->stream), "small buffer");
-            check(cudaMallocHost(reinterpret_cast<void**>(&hp->host_small), 256), "pinned buffer");
+            check(cudaMallocHost(reinterpret_cast<void**>(&hp->host_small), kHostSmallBytes), "pinned buffer");
             check(cudaMalloc(&hp->table, kTableBytes), "lattice table");
         };
         std::size_t free_bytes = 0, total_bytes = 0;
@@ -568,25 +568,26 @@ orr_status orr_lbm3d_force(orr_lbm3d* solver, double force_moment[6]) {
             throw Refusal{ORR_ERR_INVALID, "null output"};
         }
         const std::size_t links = h->plan.link_cell.size();
-        check(h->ops->force(h->g, h->f[h->cur], h->lcell, h->ldir, h->lq, links, h->acc(), h->stream),
-              "force kernel");
-        if (links > 0) {
-            ++h->launches;
+        if (links == 0) {
+            h->check_status();
+            check(cudaStreamSynchronize(h->stream), "force read-back");
+            std::fill_n(force_moment, 6, 0.0);
+            return ORR_OK;
         }
-        // One read-back: the six sums (64 bytes into the small buffer) and,
-        // for the persistent step, its status word (kStatusOffset).
-        static_assert(kStatusOffset >= 64 + 6 * sizeof(double) && kStatusOffset + 4 <= 64 + 192);
+        // The kernel writes the six sums, and the persistent step's status
+        // word after them, to the pinned buffer itself.
         const bool watched = h->persistent || h->tiled;
-        const std::size_t bytes = watched ? kStatusOffset + 4 - 64 : 6 * sizeof(double);
-        check(cudaMemcpyAsync(h->host_small + 8, h->acc(), bytes, cudaMemcpyDeviceToHost, h->stream),
-              "force read-back");
+        check(h->ops->force(h->g, h->f[h->cur], h->lcell, h->ldir, h->lq, links, h->force_scratch(),
+                            h->host_small + kHostForce, watched ? h->status() : nullptr, h->stream),
+              "force kernel");
+        ++h->launches;
         check(cudaStreamSynchronize(h->stream), "force read-back");
         if (watched) {
             uint32_t word = 0;
-            std::memcpy(&word, reinterpret_cast<const char*>(h->host_small + 8) + (kStatusOffset - 64), 4);
+            std::memcpy(&word, h->host_small + kHostForce + 6, 4);
             orr_lbm3d::raise_status(word);
         }
-        std::memcpy(force_moment, h->host_small + 8, 6 * sizeof(double));
+        std::memcpy(force_moment, h->host_small + kHostForce, 6 * sizeof(double));
         return ORR_OK;
     });
 }

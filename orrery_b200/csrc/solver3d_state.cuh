@@ -14,8 +14,8 @@
 //   moments       4 planes (rho or rho - 1, ux, uy, uz) for read-back
 //   history       5 * ny * nz convective-outlet values, twice (a step reads one and
 //                 writes the other; one copy for the zero-gradient outlet)
-//   small         force/moment (6) and mass accumulators, the inlet velocity and its
-//                 absorbing targets,
+//   small         mass accumulator, the inlet velocity and its absorbing targets, the
+//                 force kernel's scratch,
 //                 the persistent step's status word
 //   table         the lattice-table entry of the persistent step
 // Steps run as CUDA graphs of kGraphSteps steps, one kernel launch each:
@@ -55,8 +55,12 @@ constexpr uint32_t kGraphSteps = 16; // even: a graph returns to the buffer it s
 constexpr uint32_t kDefaultBlock = 128;
 constexpr std::size_t kStatusOffset = 128; // bytes into the small buffer
 constexpr std::size_t kInletOffset = 256;
-constexpr std::size_t kSmallBytes = 512;
-static_assert(kInletOffset + kInletValues * sizeof(double) <= kSmallBytes);
+constexpr std::size_t kForceOffset = 512;
+constexpr std::size_t kSmallBytes = 16384;
+constexpr std::size_t kHostForce = 32;       // values into the pinned buffer
+constexpr std::size_t kHostSmallBytes = 512;
+static_assert(kForceOffset + sizeof(ForceScratch) <= kSmallBytes);
+static_assert(kInletOffset + kInletValues * sizeof(double) <= kForceOffset);
 
 template <class T> T* device_alloc(std::size_t count, const char* what) {
     void* p = nullptr;
@@ -153,6 +157,9 @@ struct orr_lbm3d {
     void* inlet_dev() const { return static_cast<char*>(small) + kInletOffset; }
     uint32_t* status() const {
         return reinterpret_cast<uint32_t*>(static_cast<char*>(small) + kStatusOffset);
+    }
+    ForceScratch* force_scratch() const {
+        return reinterpret_cast<ForceScratch*>(static_cast<char*>(small) + kForceOffset);
     }
     double* acc() const { return reinterpret_cast<double*>(static_cast<char*>(small) + 64); }
 
