@@ -210,7 +210,7 @@ orr_status orr_gl2d_step(orr_gl2d* tables, const orr_gl2d_params* params, const 
         const Phys2D<float> phys = phys_of2(*params);
         const StepBuffers2D b{t->cls, t->nmask, {outlet, outlet}};   // the driver's one history, in place
         const bool smag = params->smagorinsky_c2 > 0.0f;
-        check(ops2d_f32().step(t->g, &phys, src, dst, b, smag, 128u, static_cast<cudaStream_t>(stream)),
+        check(ops2d_f32().step(t->g, &phys, src, dst, b, smag, 128u, false, static_cast<cudaStream_t>(stream)),
               "gl2d step kernel");
         return ORR_OK;
     });

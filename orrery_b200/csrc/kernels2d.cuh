@@ -291,11 +291,12 @@ template <class S> constexpr int kStep2dMinBlocks = sizeof(typename Storage<S>::
 
 template <class S, bool kSmag, class O>
 __global__ void __launch_bounds__(256, kStep2dMinBlocks<S>)
-    step2d_kernel(Geom2D g, Phys2D<typename Storage<S>::A> p, const S* __restrict__ src, S* __restrict__ dst,
+    step2d_kernel(Geom2D g, Phys2D<typename Storage<S>::A> p, const S* src, S* __restrict__ dst,
                   LinearOffsets2D<O> l, StepBuffers2D b, FastDiv by_nx) {
     using A = typename Storage<S>::A;
     using T = Storage<S>;
-    const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    after_last_step<S>(h);
     if (h >= static_cast<uint32_t>(g.cells)) {
         return;
     }

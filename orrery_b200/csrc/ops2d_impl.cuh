@@ -11,7 +11,7 @@ namespace orr {
 template <class S> struct Launch2D {
     using A = typename Storage<S>::A;
     static cudaError_t step(const Geom2D& g, const void* phys, const void* src, void* dst,
-                            const StepBuffers2D& b, bool smag, uint32_t block, cudaStream_t s) {
+                            const StepBuffers2D& b, bool smag, uint32_t block, bool chained, cudaStream_t s) {
         const unsigned blocks = static_cast<unsigned>((g.cells + block - 1) / block);
         const auto& p = *static_cast<const Phys2D<A>*>(phys);
         const auto launch = [&]<class O>() {
@@ -24,17 +24,15 @@ template <class S> struct Launch2D {
             }
             l.last = static_cast<O>((d2::Q * g.cells - 1) * sizeof(S));
             const auto kernel = smag ? &step2d_kernel<S, true, O> : &step2d_kernel<S, false, O>;
-            kernel<<<blocks, block, 0, s>>>(g, p, static_cast<const S*>(src), static_cast<S*>(dst), l, b,
-                                            fast_div(g.nx));
+            return launch_step<S>(kernel, blocks, block, chained, s, g, p, static_cast<const S*>(src),
+                               static_cast<S*>(dst), l, b, fast_div(g.nx));
         };
         // Past the buffer's end by at most a row before it is held: the sums
         // must not wrap.
         if ((d2::Q * g.cells + g.nx) * sizeof(S) <= 0xffffffffull) {
-            launch.template operator()<uint32_t>();
-        } else {
-            launch.template operator()<uint64_t>();
+            return launch.template operator()<uint32_t>();
         }
-        return cudaGetLastError();
+        return launch.template operator()<uint64_t>();
     }
 
     static cudaError_t init(const Geom2D& g, const uint8_t* cls, const double* rho,

@@ -21,9 +21,11 @@ struct Ops3D {
     // the storage's arithmetic type; `block` is the block width (threads
     // along x of a row, or of a linear tile where step_linear says so); npt 2
     // takes the pair step (two neighbouring nodes per thread) where pairs_ok
-    // allows it, the one-node step otherwise.
+    // allows it, the one-node step otherwise.  chained: the launch before it on
+    // the stream is the same solver's step (the one-node steps overlap its end).
     cudaError_t (*step)(const Geom3D& g, const void* phys, const void* src, void* dst,
-                        const StepBuffers3D& b, bool smag, uint32_t block, uint32_t npt, cudaStream_t s);
+                        const StepBuffers3D& b, bool smag, uint32_t block, uint32_t npt, bool chained,
+                        cudaStream_t s);
     // Equilibrium initialisation of a population buffer; rho..uz may be
     // device arrays (all non-null) or null for the uniform state (r0, u0).
     cudaError_t (*init)(const Geom3D& g, const uint8_t* cls, const double* rho, const double* ux,

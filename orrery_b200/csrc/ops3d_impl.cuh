@@ -15,7 +15,8 @@ template <class S> struct Launch3D {
     using A = typename Storage<S>::A;
 
     static cudaError_t step(const Geom3D& g, const void* phys, const void* src, void* dst,
-                            const StepBuffers3D& b, bool smag, uint32_t block, uint32_t npt, cudaStream_t s) {
+                            const StepBuffers3D& b, bool smag, uint32_t block, uint32_t npt, bool chained,
+                            cudaStream_t s) {
         Geom3D gg = g;
         gg.tiles_x = (g.nx + block - 1) / block;
         const auto& p = *static_cast<const Phys3D<A>*>(phys);
@@ -44,31 +45,26 @@ template <class S> struct Launch3D {
                     l.out[i] = static_cast<uint32_t>(to * static_cast<int64_t>(sizeof(S)));
                 }
                 const unsigned blocks = static_cast<unsigned>((g.cells + block - 1) / block);
-                linear_kernel(smag)<<<blocks, block, 0, s>>>(gg, p, in, out, l, b,
-                                                             LinearDivs3D{fast_div(g.nx), fast_div(g.ny)});
-                return cudaGetLastError();
+                return launch_step<S>(linear_kernel(smag), blocks, block, chained, s, gg, p, in, out, l, b,
+                                   LinearDivs3D{fast_div(g.nx), fast_div(g.ny)});
             }
         }
         const dim3 grid(gg.tiles_x, g.ny, g.nz);
         const auto launch = [&]<bool K>() {
             if (g.flat) {
-                step3d_kernel<S, K, Walls::Halfway><<<grid, block, 0, s>>>(gg, p, in, out, b);
-            } else if (g.open) {
+                return launch_step<S>(&step3d_kernel<S, K, Walls::Halfway>, grid, block, chained, s, gg, p, in, out, b);
+            }
+            if (g.open) {
                 StepBuffers3D w = b;
                 const uint64_t layer = static_cast<uint64_t>(gg.tiles_x) * g.ny * block;
                 w.wall_layers = static_cast<uint32_t>((b.wall_count + layer - 1) / layer);
                 const dim3 with_walls(gg.tiles_x, g.ny, g.nz + w.wall_layers);
-                step3d_kernel<S, K, Walls::Interpolated><<<with_walls, block, 0, s>>>(gg, p, in, out, w);
-            } else {
-                step3d_kernel<S, K, Walls::General><<<grid, block, 0, s>>>(gg, p, in, out, b);
+                return launch_step<S>(&step3d_kernel<S, K, Walls::Interpolated>, with_walls, block, chained, s, gg, p, in,
+                                   out, w);
             }
+            return launch_step<S>(&step3d_kernel<S, K, Walls::General>, grid, block, chained, s, gg, p, in, out, b);
         };
-        if (smag) {
-            launch.template operator()<true>();
-        } else {
-            launch.template operator()<false>();
-        }
-        return cudaGetLastError();
+        return smag ? launch.template operator()<true>() : launch.template operator()<false>();
     }
 
     // The linear order serves flat lattices whose buffers 32-bit byte offsets

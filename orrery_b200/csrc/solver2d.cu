@@ -88,9 +88,9 @@ struct orr_lbm2d {
         if (stream) cudaStreamDestroy(stream);
     }
 
-    void launch_step(int from) {
+    void launch_step(int from, bool chained = false) {
         const StepBuffers2D b = buffers(from);
-        check(ops->step(g, phys(), f[from], f[1 - from], b, smag, block, stream), "step kernel");
+        check(ops->step(g, phys(), f[from], f[1 - from], b, smag, block, chained, stream), "step kernel");
         ++launches;
     }
 
@@ -101,7 +101,7 @@ struct orr_lbm2d {
         check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "graph capture");
         try {
             for (uint32_t k = 0; k < kGraphSteps2; ++k) {
-                launch_step(static_cast<int>(k & 1u));
+                launch_step(static_cast<int>(k & 1u), k > 0);
             }
         } catch (...) {
             cudaStreamEndCapture(stream, &captured);
@@ -133,8 +133,8 @@ struct orr_lbm2d {
                 left -= kGraphSteps2;
             }
         }
-        for (; left > 0; --left) {
-            launch_step(cur);
+        for (bool chained = false; left > 0; --left, chained = true) {
+            launch_step(cur, chained);
             cur = 1 - cur;
         }
         steps += count;

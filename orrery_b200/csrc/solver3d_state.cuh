@@ -224,8 +224,9 @@ struct orr_lbm3d {
         check(cudaStreamSynchronize(stream), "inlet upload");
     }
 
-    // One step src -> dst on `stream` (one kernel launch).
-    void launch_step(int from) {
+    // One step src -> dst on `stream` (one kernel launch); chained: this
+    // function made the launch before it.
+    void launch_step(int from, bool chained = false) {
         if (tiled) {
             check(ops->tiled(host_table, tmaps, tgrid, static_cast<uint32_t>(from), shape.stages, smag, tile_rows,
                              shape.block, shape.grid, status(), stream),
@@ -235,7 +236,7 @@ struct orr_lbm3d {
                               shape.stages, smag, shape.block, shape.npt, shape.grid, status(), stream),
                   "step kernel");
         } else {
-            check(ops->step(g, phys(), f[from], f[1 - from], buffers(from), smag, block, row_npt, stream),
+            check(ops->step(g, phys(), f[from], f[1 - from], buffers(from), smag, block, row_npt, chained, stream),
                   "step kernel");
         }
         ++launches;
@@ -283,7 +284,7 @@ struct orr_lbm3d {
         const uint64_t before = launches;
         try {
             for (uint32_t k = 0; k < kGraphSteps; ++k) {
-                launch_step(static_cast<int>(k & 1u));
+                launch_step(static_cast<int>(k & 1u), k > 0);
             }
         } catch (...) {
             cudaStreamEndCapture(stream, &captured);
@@ -315,8 +316,8 @@ struct orr_lbm3d {
                 left -= kGraphSteps;
             }
         }
-        for (; left > 0; --left) {
-            launch_step(cur);
+        for (bool chained = false; left > 0; --left, chained = true) {
+            launch_step(cur, chained);
             cur = 1 - cur;
         }
         steps += count;
