@@ -16,6 +16,14 @@ struct Geom3D;
 struct StepBuffers3D;
 struct ForceScratch;
 
+// Threads per block of the linear-order step where the caller names none: 256
+// from 5.5 million nodes on, 128 below.  us per step with 128 and 256, binary16
+// and binary32, convective outlet: 112 x 56 x 56 13.2 13.9, 11.1 12.1; 240 x 120 x
+// 120 68.5 70.0, 87.5 88.3; 272 x 136 x 136 (5.0 million) 97.4 97.5, 124.9 125.2;
+// 300 x 150 x 150 (6.8 million) 135.7 127.8, 165.6 165.4; 400 x 200 x 200 340 293,
+// 382 379; 512 x 256 x 256 692 589 (binary16).
+inline uint32_t linear_block(uint64_t cells) { return cells >= 5500000u ? 256u : 128u; }
+
 struct Ops3D {
     // One fused step src -> dst (one launch).  `phys` points at a Phys3D of
     // the storage's arithmetic type; `block` is the block width (threads

@@ -468,9 +468,7 @@ orr_status orr_lbm3d_create(const orr_lbm3d_config* config, const uint8_t* solid
             }
             h->row_npt = 2;
         } else if (o.block_x == 0 && h->ops->step_linear(g)) {
-            // Linear tiles of 256 nodes: binary16 512 x 256 x 256 takes 566 us
-            // per step with 256, 668 with 128; small lattices the same.
-            h->block = 256u;
+            h->block = linear_block(g.cells);
         }
         initialize_state(h.get(), nullptr, nullptr, nullptr, nullptr);
         // Capture the step graph now, so that no step() call, the first

@@ -59,3 +59,18 @@ def test_interpolated_walls_within_rounding(size, storage, eps):
     want = populations((c, mask), state, "f64")
     got = populations((c, mask), state, storage)
     assert np.max(np.abs(got - want)) < 19 * 2 * 0.04 * max(eps, 2.0 ** -22)
+
+
+# The default tile changes at 5.5 million nodes: equal bits on both sides of it.
+@pytest.mark.parametrize("nz,block", [(134, 128), (135, 256)])
+def test_default_tile(nz, block):
+    c, mask, _ = lattice((300, 136, nz), WallKind.slip, XBoundary.inflow_outflow, SolidWall.halfway, True)
+    fields = []
+    for options in ({}, {"block_x": 64}):
+        s = S.make_gpu_solver(c, mask, storage="f16", **options)
+        assert s.kernel_info()["block"] == options.get("block_x", block)
+        s.step(5)
+        m = s.macroscopic()
+        fields.append([m.density, m.velocity_x, m.velocity_y, m.velocity_z])
+        s.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*fields))
