@@ -469,6 +469,8 @@ orr_status orr_lbm3d_create(const orr_lbm3d_config* config, const uint8_t* solid
             h->row_npt = 2;
         } else if (o.block_x == 0 && h->ops->step_linear(g)) {
             h->block = linear_block(g.cells);
+        } else if (o.block_x == 0 && !binary32 && g.open && one_warp_rows(g.nx, g.ny, g.nz)) {
+            h->block = 32u;
         }
         initialize_state(h.get(), nullptr, nullptr, nullptr, nullptr);
         // Capture the step graph now, so that no step() call, the first
