@@ -1223,8 +1223,10 @@ inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, uint32_t block, 
 // of row (y, z).  b.hist[0] is the source buffer's history.
 // kWalls: Halfway for lattices with g.flat set, Interpolated for those with
 // g.open only, General for the others.
-template <class S, bool kSmag, Walls kWalls>
-__global__ void __launch_bounds__(256, kStepMinBlocks<S, kWalls>)
+// kDense: blocks of at most 128 threads, five of them an SM (96 registers instead
+// of 122), for binary64 with halfway walls (dense_rows in the launcher).
+template <class S, bool kSmag, Walls kWalls, bool kDense = false>
+__global__ void __launch_bounds__(kDense ? 128 : 256, kDense ? 5 : kStepMinBlocks<S, kWalls>)
     step3d_kernel(Geom3D g, Phys3D<typename Storage<S>::A> p, const S* src, S* __restrict__ dst, StepBuffers3D b) {
     uint32_t z = blockIdx.z;
     uint32_t lane = threadIdx.x;

@@ -25,7 +25,8 @@ struct ForceScratch;
 inline uint32_t linear_block(uint64_t cells) { return cells >= 5500000u ? 256u : 128u; }
 
 // Whether the binary64 row step of an open lattice takes one-warp blocks where
-// the caller names none.  Its blocks are limited by registers (16 warps an SM),
+// the caller names none.  Its blocks are limited by registers (16 or 20 warps an
+// SM; the figures are with 16),
 // and the warps of a 128-node tile beyond the row's end keep theirs until the
 // tile is done: one-warp blocks have none.  They start later, so tiles stay where
 // a wave holds them all (4 an SM, 148 SMs) or the rows are short and leave
@@ -66,7 +67,7 @@ struct Ops3D {
     // Whether the one-node step of lattice g runs in linear order.
     bool (*step_linear)(const Geom3D& g);
     // Registers per thread of lattice g's step kernel.
-    int (*step_registers)(const Geom3D& g, bool smag, uint32_t npt);
+    int (*step_registers)(const Geom3D& g, bool smag, uint32_t block, uint32_t npt);
     // Whether the pair step serves lattice g with blocks of `block` threads
     // (2-byte storage, periodic or free-slip sides and halfway walls, even nx,
     // whole warps up to 128 threads).

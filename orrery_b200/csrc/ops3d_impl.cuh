@@ -52,6 +52,12 @@ template <class S> struct Launch3D {
         const dim3 grid(gg.tiles_x, g.ny, g.nz);
         const auto launch = [&]<bool K>() {
             if (g.flat) {
+                if constexpr (sizeof(A) == 8) {
+                    if (dense_rows(g, block)) {
+                        return launch_step<S>(&step3d_kernel<S, K, Walls::Halfway, true>, grid, block, chained, s, gg,
+                                              p, in, out, b);
+                    }
+                }
                 return launch_step<S>(&step3d_kernel<S, K, Walls::Halfway>, grid, block, chained, s, gg, p, in, out, b);
             }
             if (g.open) {
@@ -65,6 +71,17 @@ template <class S> struct Launch3D {
             return launch_step<S>(&step3d_kernel<S, K, Walls::General>, grid, block, chained, s, gg, p, in, out, b);
         };
         return smag ? launch.template operator()<true>() : launch.template operator()<false>();
+    }
+
+    // The binary64 step waits on memory and long arithmetic with 16 warps an SM;
+    // 20 at 96 registers hide more of both for some spilled values: us per
+    // step, 256 x 128 x 128 274 -> 259, 128 x 64 x 64 44.4 -> 41.4, 337 x 193 x 193 780 -> 765.
+    // Where 16 warps an SM hold the lattice the spills are all that changes
+    // (64 x 32 x 32 8.1 -> 8.4), interpolated walls spill far more (337 x 193 x 193
+    // 806 -> 827), and 24 warps at 80 registers are slower (256 x 128 x 128 305).
+    static bool dense_rows(const Geom3D& g, uint32_t block) {
+        return sizeof(A) == 8 && g.flat && block <= 128 &&
+               static_cast<uint64_t>((g.nx + 31) / 32) * g.ny * g.nz > 148u * 16u;
     }
 
     // The linear order serves flat lattices whose buffers 32-bit byte offsets
@@ -131,7 +148,7 @@ template <class S> struct Launch3D {
         return sizeof(S) == 2 && g.flat && g.nx % 2 == 0 && block % 32 == 0 && block <= 128;
     }
 
-    static int step_registers(const Geom3D& g, bool smag, uint32_t npt) {
+    static int step_registers(const Geom3D& g, bool smag, uint32_t block, uint32_t npt) {
         cudaFuncAttributes a{};
         const auto registers = [&a](auto kernel) {
             return cudaFuncGetAttributes(&a, kernel) == cudaSuccess ? a.numRegs : -1;
@@ -144,6 +161,12 @@ template <class S> struct Launch3D {
         if constexpr (sizeof(A) == 4) {
             if (step_linear(g)) {
                 return registers(linear_kernel(smag));
+            }
+        }
+        if constexpr (sizeof(A) == 8) {
+            if (dense_rows(g, block)) {
+                return registers(smag ? &step3d_kernel<S, true, Walls::Halfway, true>
+                                      : &step3d_kernel<S, false, Walls::Halfway, true>);
             }
         }
         const auto of = [&]<Walls K>() {

@@ -6,7 +6,8 @@ import pytest
 from helpers import Outlet
 from orrery_b200 import masks as M
 from orrery_b200 import solver as S
-from orrery_b200.lbm3d import Lbm3DConfig, SolidWall, WallKind, XBoundary, wall
+from orrery_b200.lbm3d import Lbm3DConfig, Smagorinsky, SolidWall, WallKind, XBoundary, wall
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +31,23 @@ def test_default_tile(size, sides, block, solid_wall):
         got.append(s.populations())
         s.close()
     assert np.array_equal(*got)
+
+
+# The 96-register form (halfway walls, blocks up to 128, more than 2,368 warps
+# of rows) and the plain one have the oracle's bits.
+@pytest.mark.parametrize("size,block,dense", [((32, 74, 32), 0, False), ((32, 75, 32), 0, True), ((97, 25, 24), 128, True),
+                                              ((97, 25, 24), 160, False), ((33, 37, 33), 96, True)])
+@pytest.mark.parametrize("les", [False, True])
+def test_dense_rows_match_the_oracle(size, block, dense, les):
+    nx, ny, nz = size
+    c = Lbm3DConfig(nx=nx, ny=ny, nz=nz, tau=0.55, x_boundary=XBoundary.inflow_outflow, outlet=Outlet.convective,
+                    y_low=wall(WallKind.slip), y_high=wall(WallKind.slip), z_low=wall(WallKind.periodic),
+                    z_high=wall(WallKind.periodic), inlet_ux=0.05, smagorinsky=Smagorinsky(les, 0.1))
+    mask = M.sphere_mask(nx, ny, nz, (nx / 3.0, 0.4, nz / 2.0), nz / 5.0)
+    ref, s = O.Restated3D(c, mask.solid), S.make_gpu_solver(c, mask, storage="f64", block_x=block)
+    assert (s.kernel_info()["registers"] <= 96) == dense
+    ref.initialize()
+    s.initialize()
+    ref.step(19)
+    s.step(19)
+    assert np.array_equal(s.populations(), ref.populations())
