@@ -26,14 +26,13 @@ inline uint32_t linear_block(uint64_t cells) { return cells >= 5500000u ? 256u :
 
 // Whether the binary64 row step of an open lattice takes one-warp blocks where
 // the caller names none.  Its blocks are limited by registers (16 or 20 warps an
-// SM; the figures are with 16),
-// and the warps of a 128-node tile beyond the row's end keep theirs until the
-// tile is done: one-warp blocks have none.  They start later, so tiles stay where
-// a wave holds them all (4 an SM, 148 SMs) or the rows are short and leave
-// one warp idle.  us per step with 128 and 32 nodes, halfway walls: nx 64 10.3
-// 8.1, 160 85.0 76.3, 200 158 145, 300 471 426, 337 634 590 (ny = nz = nx / 2); not
-// taken: 40 6.3 6.6, 80 14.7 14.7 (interpolated walls 14.9 15.2), 97 21.8 24.0, 128 64 64
-// 38.3 39.3.
+// SM; the figures are with 16), and the warps of a 128-node tile beyond the row's
+// end keep theirs until the tile is done: one-warp blocks have none.  They start
+// later, so tiles stay where a wave holds them all (4 an SM, 148 SMs) or the rows
+// are short and leave one warp idle.  us per step with 128 and 32 nodes, halfway
+// walls: nx 64 10.3 8.1, 160 85.0 76.3, 200 158 145, 300 471 426, 337 634 590 (ny =
+// nz = nx / 2); not taken: 40 6.3 6.6, 80 14.7 14.7 (interpolated walls 14.9 15.2),
+// 97 21.8 24.0, 128 x 64 x 64 38.3 39.3.
 inline bool one_warp_rows(uint64_t nx, uint64_t ny, uint64_t nz) {
     const uint64_t idle = (4u - (nx + 31u) / 32u % 4u) % 4u;   // warps of the last tile
     return (nx > 128u ? idle > 0u : idle >= 2u) && (nx + 127u) / 128u * ny * nz > 4u * 148u;

@@ -75,7 +75,7 @@ template <class S> struct Launch3D {
 
     // The binary64 step waits on memory and long arithmetic with 16 warps an SM;
     // 20 at 96 registers hide more of both for some spilled values: us per
-    // step, 256 x 128 x 128 274 -> 259, 128 x 64 x 64 44.4 -> 41.4, 337 x 193 x 193 780 -> 765.
+    // step with the convective outlet, 256 x 128 x 128 274 -> 259, 128 x 64 x 64 44.4 -> 41.4, 337 x 193 x 193 780 -> 765.
     // Where 16 warps an SM hold the lattice the spills are all that changes
     // (64 x 32 x 32 8.1 -> 8.4), interpolated walls spill far more (337 x 193 x 193
     // 806 -> 827), and 24 warps at 80 registers are slower (256 x 128 x 128 305).
