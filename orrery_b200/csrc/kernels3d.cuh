@@ -18,6 +18,7 @@
 #include <cstdint>
 #include <initializer_list>
 
+#include "fast_div.h"
 #include "lattice.h"
 #include "orrery_lbm.h"
 #include "storage.cuh"
@@ -1248,26 +1249,6 @@ __global__ void __launch_bounds__(kDense ? 128 : 256, kDense ? 5 : kStepMinBlock
     }
     step_node3<S, kSmag, kWalls>(g, p, src, dst, b, x, blockIdx.y, z, 0u);
 }
-
-// Quotients n / d of 32-bit n < 2^31 by multiplication.
-struct FastDiv {
-    uint32_t mul = 0, shift = 0;
-};
-inline FastDiv fast_div(uint32_t d) {
-    // mul = ceil(2^(32 + shift) / d) with 2^shift <= d < 2^(shift + 1): mul d
-    // exceeds 2^(32 + shift) by less than d, so n mul / 2^(32 + shift) is below
-    // n / d + 1 / d while n < 2^31.  A power of two takes half of both.
-    FastDiv f;
-    while ((d >> f.shift) > 1u) ++f.shift;
-    if ((d & (d - 1u)) == 0u) {
-        f.mul = d == 1u ? 0xffffffffu : 1u << 31;
-        f.shift = d == 1u ? 0u : f.shift - 1u;
-    } else {
-        f.mul = static_cast<uint32_t>(((uint64_t{1} << (32 + f.shift)) + d - 1u) / d);
-    }
-    return f;
-}
-__device__ __forceinline__ uint32_t divide(uint32_t n, FastDiv f) { return __umulhi(n, f.mul) >> f.shift; }
 
 // Byte offsets of direction i's pull and store of node 0 from the population
 // buffers.
