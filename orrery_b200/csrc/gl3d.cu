@@ -169,17 +169,29 @@ __global__ void gl_link_force_kernel(Geom3D g, const float* __restrict__ f, cons
     }
 }
 
-// Uploads the inlet velocity when it changed since the last dispatch.
+// The inlet values as a kernel argument: a launch holds its own copy, also in a
+// captured graph, which would read a host buffer at each replay.
+struct InletValues {
+    float v[kInletValues];
+};
+
+__global__ void store_inlet_kernel(InletValues in, float* __restrict__ to) {
+    if (threadIdx.x < kInletValues) {
+        to[threadIdx.x] = in.v[threadIdx.x];
+    }
+}
+
+// Writes the inlet velocity when it changed since the last dispatch.
 void sync_inlet(orr_gl3d* t, const orr_gl3d_params& p, cudaStream_t s) {
     if (t->inlet_set && std::memcmp(t->inlet_host, p.inlet, sizeof t->inlet_host) == 0) {
         return;
     }
     std::memcpy(t->inlet_host, p.inlet, sizeof t->inlet_host);
-    // From pageable memory: the call returns once the values are staged.
     const double v[3] = {p.inlet[0], p.inlet[1], p.inlet[2]};
-    float values[kInletValues];
-    fill_inlet(values, v);
-    check(cudaMemcpyAsync(t->inlet, values, sizeof values, cudaMemcpyHostToDevice, s), "gl3d inlet");
+    InletValues values;
+    fill_inlet(values.v, v);
+    store_inlet_kernel<<<1, 32, 0, s>>>(values, t->inlet);
+    check(cudaGetLastError(), "gl3d inlet");
     t->inlet_set = true;
 }
 
