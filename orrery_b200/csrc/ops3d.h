@@ -65,8 +65,8 @@ struct Ops3D {
                         cudaStream_t s);
     // Whether the one-node step of lattice g runs in linear order.
     bool (*step_linear)(const Geom3D& g);
-    // Registers per thread of lattice g's step kernel.
-    int (*step_registers)(const Geom3D& g, bool smag, uint32_t block, uint32_t npt);
+    // Registers per thread of lattice g's step kernel (wall_count: StepBuffers3D's).
+    int (*step_registers)(const Geom3D& g, bool smag, uint32_t block, uint32_t npt, uint32_t wall_count);
     // Whether the pair step serves lattice g with blocks of `block` threads
     // (2-byte storage, periodic or free-slip sides and halfway walls, even nx,
     // whole warps up to 128 threads).

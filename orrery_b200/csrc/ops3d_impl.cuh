@@ -60,10 +60,9 @@ template <class S> struct Launch3D {
                 }
                 return launch_step<S>(&step3d_kernel<S, K, Walls::Halfway>, grid, block, chained, s, gg, p, in, out, b);
             }
-            if (g.open) {
+            if (walls_listed(g, block, b.wall_count)) {
                 StepBuffers3D w = b;
-                const uint64_t layer = static_cast<uint64_t>(gg.tiles_x) * g.ny * block;
-                w.wall_layers = static_cast<uint32_t>((b.wall_count + layer - 1) / layer);
+                w.wall_layers = wall_layers(g, block, b.wall_count);
                 const dim3 with_walls(gg.tiles_x, g.ny, g.nz + w.wall_layers);
                 return launch_step<S>(&step3d_kernel<S, K, Walls::Interpolated>, with_walls, block, chained, s, gg, p, in,
                                    out, w);
@@ -71,6 +70,19 @@ template <class S> struct Launch3D {
             return launch_step<S>(&step3d_kernel<S, K, Walls::General>, grid, block, chained, s, gg, p, in, out, b);
         };
         return smag ? launch.template operator()<true>() : launch.template operator()<false>();
+    }
+
+    // Layers of the grid that hold the wall list's blocks, in front of the rows'.
+    static uint32_t wall_layers(const Geom3D& g, uint32_t block, uint32_t wall_count) {
+        const uint64_t layer = static_cast<uint64_t>((g.nx + block - 1) / block) * g.ny * block;
+        return static_cast<uint32_t>((wall_count + layer - 1) / layer);
+    }
+
+    // Whether an open lattice's interpolated walls are stepped from their list.
+    // The layers share the grid's z with the rows: a lattice whose nz leaves them no
+    // room takes the general node code.
+    static bool walls_listed(const Geom3D& g, uint32_t block, uint32_t wall_count) {
+        return g.open && !g.flat && uint64_t{g.nz} + wall_layers(g, block, wall_count) <= 65535u;
     }
 
     // The binary64 step waits on memory and long arithmetic with 16 warps an SM;
@@ -148,7 +160,7 @@ template <class S> struct Launch3D {
         return sizeof(S) == 2 && g.flat && g.nx % 2 == 0 && block % 32 == 0 && block <= 128;
     }
 
-    static int step_registers(const Geom3D& g, bool smag, uint32_t block, uint32_t npt) {
+    static int step_registers(const Geom3D& g, bool smag, uint32_t block, uint32_t npt, uint32_t wall_count) {
         cudaFuncAttributes a{};
         const auto registers = [&a](auto kernel) {
             return cudaFuncGetAttributes(&a, kernel) == cudaSuccess ? a.numRegs : -1;
@@ -172,9 +184,9 @@ template <class S> struct Launch3D {
         const auto of = [&]<Walls K>() {
             return registers(smag ? &step3d_kernel<S, true, K> : &step3d_kernel<S, false, K>);
         };
-        return g.flat   ? of.template operator()<Walls::Halfway>()
-               : g.open ? of.template operator()<Walls::Interpolated>()
-                        : of.template operator()<Walls::General>();
+        return g.flat                                ? of.template operator()<Walls::Halfway>()
+               : walls_listed(g, block, wall_count) ? of.template operator()<Walls::Interpolated>()
+                                                     : of.template operator()<Walls::General>();
     }
 
     template <bool kSmag, int B, int NPT, bool kSingle> static constexpr auto staged_kernel() {

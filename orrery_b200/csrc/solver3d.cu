@@ -769,7 +769,8 @@ orr_status orr_lbm3d_kernel_info(const orr_lbm3d* solver, orr_kernel_info* info)
             k.grid = solver->row_npt == 1 && solver->ops->step_linear(solver->g)
                          ? static_cast<uint32_t>((solver->g.cells + span - 1) / span)
                          : ((solver->g.nx + span - 1) / span) * solver->g.ny * solver->g.nz;
-            k.registers = solver->ops->step_registers(solver->g, solver->smag, solver->block, solver->row_npt);
+            k.registers = solver->ops->step_registers(solver->g, solver->smag, solver->block, solver->row_npt,
+                                                      solver->wall_count);
         }
         *info = k;
         return ORR_OK;
