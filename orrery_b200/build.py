@@ -4,7 +4,9 @@ Every CUDA translation unit is compiled by nvcc for sm_100a only
 (``-gencode arch=compute_100a,code=sm_100a``), host C++ with the same nvcc
 driver, and the objects are linked into one shared library with the CUDA
 runtime linked statically.  The binary64 kernel unit is compiled with
-``-fmad=false`` so its arithmetic rounds like the reference CPU solver.
+``-fmad=false`` so its arithmetic rounds like the reference CPU solver; host
+code is compiled without contraction, so values formed on both sides (the
+absorbing layers' targets) have the same bits whatever the host's baseline.
 
 Usage: ``python -m orrery_b200.build [--force] [--verbose]``.
 """
@@ -25,7 +27,7 @@ OBJ_DIR = os.path.join(OUT_DIR, "obj")
 LIBRARY = os.path.join(OUT_DIR, "liborrery_lbm.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-COMMON = ["-std=c++20", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden",
+COMMON = ["-std=c++20", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden,-ffp-contract=off",
           "-I", INCLUDE, "-I", CSRC]
 
 SOURCES = {
