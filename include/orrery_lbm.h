@@ -322,7 +322,9 @@ ORR_API orr_status orr_batch3d_launch_count(const orr_batch3d* batch, uint64_t* 
  * requests in arrival order while a slot is free and the admitted lattices'
  * device memory (orr_lbm3d_memory_bytes) stays within `memory_budget` - the
  * planning, allocation and upload of new solves overlap the running chunk -
- * and retires the solves that are done.  A solve samples its force every
+ * and retires the solves that are done.  Solves on the device share the
+ * closure (Smagorinsky on or off): a request with the other one waits for them,
+ * and those behind it for it.  A solve samples its force every
  * `sample_every` steps (the reference adapter's sampling,
  * lbm_aero_solver3d.cpp:385-441) and is done when the mean Cd of its last
  * window of `window` steps differs from the previous window's by less than

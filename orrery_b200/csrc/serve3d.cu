@@ -307,9 +307,9 @@ struct orr_server {
         return true;
     }
 
-    // Admits queued requests in arrival order while a slot is free and the
-    // budget holds.  A request that cannot fit even on an empty device is
-    // refused.
+    // Admits queued requests in arrival order while a slot is free, the budget
+    // holds and the closure is the members'.  A request that cannot fit even on
+    // an empty device is refused.
     void admit() {
         for (;;) {
             std::shared_ptr<Request> q;
@@ -323,8 +323,12 @@ struct orr_server {
                     return;
                 }
                 q = queue.front();
+                const bool mates = !active.empty() || !joining.empty();
+                if (mates && closure_on(q->config, opt.storage) != (active.empty() ? joining : active).front().solver->smag) {
+                    return;   // members share the closure: wait until those with the other one are done
+                }
                 if (used_bytes + q->estimate > opt.memory_budget) {
-                    if (!active.empty() || !joining.empty()) {
+                    if (mates) {
                         return;   // wait for memory to free up
                     }
                     refuse = true;
@@ -503,14 +507,16 @@ struct orr_server {
                     }
                 }
                 // New solvers join between launches, in admission order.
-                for (Active& a : joining) {
-                    if (orr_batch3d_add(batch, a.solver) != ORR_OK) {
+                // A solve is in one of the two lists, also when a join is refused
+                // (shutdown destroys the solvers of both).
+                while (!joining.empty()) {
+                    if (orr_batch3d_add(batch, joining.front().solver) != ORR_OK) {
                         throw Refusal{ORR_ERR_STATE, orr_batch3d_last_error(batch)};
                     }
-                    active.push_back(a);
+                    active.push_back(joining.front());
+                    joining.erase(joining.begin());
                     loop_stale = true;
                 }
-                joining.clear();
                 if (active.empty()) {
                     orr::Zone zone("serve_admit");
                     admit();

@@ -347,8 +347,7 @@ orr_status orr_lbm3d_create(const orr_lbm3d_config* config, const uint8_t* solid
         }
         fill_phys(h->phys32, *config, true);
         fill_phys(h->phys64, *config, false);
-        h->smag = config->smagorinsky_enabled != 0 &&
-                  (binary32 ? h->phys32.smag_c2 > 0.0f : true);
+        h->smag = closure_on(*config, o.storage);
         // Streams and device tables (the plan-sized ones here; the others
         // unless the helper made them).
         if (h->stream == nullptr) {

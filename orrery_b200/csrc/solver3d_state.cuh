@@ -91,6 +91,13 @@ inline float to_f32(double v) {
     return static_cast<float>(v);
 }
 
+// Whether a solver of this configuration runs the Smagorinsky closure (its
+// squared constant may round to zero in binary32).
+inline bool closure_on(const orr_lbm3d_config& c, int32_t storage) {
+    return c.smagorinsky_enabled != 0 &&
+           (storage == ORR_STORAGE_F64 || to_f32(c.smagorinsky_constant * c.smagorinsky_constant) > 0.0f);
+}
+
 } // namespace orr
 
 // (A private header of this library: the handle is a global C type.)
