@@ -576,7 +576,7 @@ std::optional<std::size_t> memory3d(const orr_lbm3d_config& c, std::size_t links
     // Links: cell, direction, fraction.
     if (!mul(links, 16, t) || !add(total, t, total)) return std::nullopt;
     // Force, mass and inlet buffers; slack of the staged step; table entry.
-    if (!add(total, 16384 + 4 * kPopPad * s + kClassPad + kTableBytes, total)) return std::nullopt;
+    if (!add(total, 65536 + 4 * kPopPad * s + kClassPad + kTableBytes, total)) return std::nullopt;
     return total;
 }
 
@@ -740,7 +740,7 @@ std::optional<std::size_t> memory2d(const orr_lbm2d_config& c, std::size_t links
     const std::size_t s = storage_bytes(storage), a = arithmetic_bytes(storage);
     return cells * (d2::Q * s * 2 + 1 + 3 * a) +
            c.ny * d2::kOutletSlots * a * (c.outlet == ORR_OUTLET_CONVECTIVE ? 2 : 1) +
-           cells * 4 + links * 8 + 16384;
+           cells * 4 + links * 8 + 65536;
 }
 
 } // namespace orr

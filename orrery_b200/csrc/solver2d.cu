@@ -27,7 +27,7 @@ using namespace orr;
 
 constexpr uint32_t kGraphSteps2 = 16;
 constexpr uint32_t kDefaultBlock2 = 128;
-constexpr std::size_t kSmallBytes2 = 16384;
+constexpr std::size_t kSmallBytes2 = 65536;
 static_assert(8 * sizeof(double) + sizeof(orr::ForceScratch) <= kSmallBytes2);
 
 const Ops2D& ops2_for(int32_t storage) {

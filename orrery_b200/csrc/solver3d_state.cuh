@@ -56,7 +56,7 @@ constexpr uint32_t kDefaultBlock = 128;
 constexpr std::size_t kStatusOffset = 128; // bytes into the small buffer
 constexpr std::size_t kInletOffset = 256;
 constexpr std::size_t kForceOffset = 512;
-constexpr std::size_t kSmallBytes = 16384;
+constexpr std::size_t kSmallBytes = 65536;
 constexpr std::size_t kHostForce = 32;       // values into the pinned buffer
 constexpr std::size_t kHostSmallBytes = 512;
 static_assert(kForceOffset + sizeof(ForceScratch) <= kSmallBytes);
