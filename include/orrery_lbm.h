@@ -596,6 +596,7 @@ ORR_API orr_status orr_lbm2d_create(const orr_lbm2d_config* config, const uint8_
 ORR_API void orr_lbm2d_destroy(orr_lbm2d* solver);
 ORR_API const char* orr_lbm2d_last_error(const orr_lbm2d* solver);
 /* Lbm2DSolver::initialize (lbm2d.h:187); rho, ux, uy arrays of nx*ny doubles
+ * (refused with ORR_ERR_INVALID, state kept, for the 2-byte population storages)
  * or all NULL for uniform_inlet_state. */
 ORR_API orr_status orr_lbm2d_initialize(orr_lbm2d* solver, const double* rho, const double* ux,
                                         const double* uy);

@@ -176,9 +176,9 @@ void initialize2(orr_lbm2d* h, const double* rho, const double* ux, const double
     if (rho != nullptr) {
         // The fields are staged in the second population buffer: three
         // binary64 planes, 24 bytes per node, where the 2-byte storages have 18.
-        // Refused before the copy: a chunk of it could start in the next allocation.
         if (3 * sizeof(double) > d2::Q * h->sbytes) {
-            throw CudaError{cudaErrorInvalidValue, "initial state upload"};
+            throw Refusal{ORR_ERR_INVALID, "lbm2d gpu: initial fields need a population storage of 4 or 8 bytes: a "
+                                           "2-byte one has no room to stage them"};
         }
         double* base = static_cast<double*>(h->f[1]);
         const double* src[3] = {rho, ux, uy};
