@@ -133,9 +133,20 @@ void widen_stripe(const Chunk& c, const unsigned char* from, std::size_t a, std:
     }
 }
 
+// A read-back's threads start while the stream's earlier work runs; the ring is
+// taken once that work is done, so that a solver in the middle of a long run
+// does not keep it from the others'.
 void staged(bool upload, const std::vector<Chunk>& chunks, cudaStream_t stream, int device) {
-    std::lock_guard<std::mutex> hold(g_ring_lock);
-    unsigned char* slots = ring();
+    std::unique_lock<std::mutex> hold(g_ring_lock, std::defer_lock);
+    unsigned char* slots = nullptr;
+    const auto take_ring = [&] {
+        check(cudaStreamSynchronize(stream), "staged copy");
+        hold.lock();
+        slots = ring();
+    };
+    if (upload) {
+        take_ring();   // the threads fill it from their start
+    }
     Events ev;
     const std::size_t n = chunks.size();
     // A small widening read-back (a 64 x 32 x 32 lattice's fields: 2 MiB)
@@ -199,6 +210,9 @@ void staged(bool upload, const std::vector<Chunk>& chunks, cudaStream_t stream, 
     try {
         for (int t = 0; t < nworkers && !alone; ++t) {
             threads.emplace_back(worker, t);
+        }
+        if (!upload) {
+            take_ring();
         }
     } catch (...) {
         pr.fail(cudaErrorUnknown, "staging threads");
