@@ -28,7 +28,8 @@ namespace {
 constexpr std::size_t kChunk = std::size_t(4) << 20;
 constexpr int kSlots = 8;
 constexpr int kMaxWorkers = 16;
-constexpr std::size_t kAloneBytes = std::size_t(4) << 20;
+constexpr std::size_t kAloneBytes = std::size_t(3) << 19;
+constexpr std::size_t kThreadBytes = std::size_t(512) << 10;
 
 // One staged copy at a time in the process: the ring is shared.  It is
 // allocated on first use (portable, so every device's DMA can use it) and
@@ -149,14 +150,19 @@ void staged(bool upload, const std::vector<Chunk>& chunks, cudaStream_t stream, 
     }
     Events ev;
     const std::size_t n = chunks.size();
-    // A small widening read-back (a 64 x 32 x 32 lattice's fields: 2 MiB)
-    // takes less time on one thread than sixteen take to start.  A larger copy
-    // keeps them all: its pages fault in faster on more threads.
+    // A thread takes about 25 us to start and moves 4 GB/s from another NUMA node's
+    // memory and 10 from its own: this thread up to kAloneBytes of host memory, then
+    // one for each kThreadBytes, up to worker_count (so only widening read-backs
+    // below 8 MiB take fewer).  us per read-back of the fields with one thread (own
+    // and other node) and sixteen: 16 x 8 x 8 40 380, 40 x 20 x 20 (0.5 MiB) 65 150 400,
+    // 56 x 28 x 28 140 360 420, 64 x 32 x 32 (2 MiB) 200 515 450, 80 x 40 x 40 360 960
+    // 500; with one per 0.5 MiB the last two 170 to 185 and 300 to 330 on its own node.
     std::size_t host_bytes = 0;
     for (const Chunk& c : chunks) {
         host_bytes += c.widen ? 2 * c.len : c.len;
     }
-    const int nworkers = host_bytes <= kAloneBytes ? 1 : worker_count(upload);
+    const std::size_t wanted = host_bytes <= kAloneBytes ? 1 : (host_bytes + kThreadBytes - 1) / kThreadBytes;
+    const int nworkers = static_cast<int>(std::min<std::size_t>(wanted, worker_count(upload)));
     Progress pr;
     pr.filled.assign(n, 0);
     const auto slot = [&](std::size_t j) { return slots + (j % kSlots) * kChunk; };

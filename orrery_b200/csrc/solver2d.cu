@@ -27,6 +27,16 @@ using namespace orr;
 
 constexpr uint32_t kGraphSteps2 = 16;
 constexpr uint32_t kDefaultBlock2 = 128;
+// Initial fields of fewer bytes are uploaded by plain copies, larger ones through
+// the staging ring, whose threads cost more than they save below.  us per
+// initialize, plain and staged: 400 x 160 111 121, 1000 x 500 (11 MiB) 645 1175,
+// 1700 x 850 1820 1880, 2048 x 1024 (48 MiB) 2390 to 2670 2320 to 2360, 3000 x 1500
+// 6230 3610.
+constexpr std::size_t kRingFields2 = std::size_t(48) << 20;
+// Binary32 populations of fewer host bytes are read by one plain copy and widened
+// here: the ring's nine planes are nine copies and as many waits (us, plain and
+// ring: 131 x 77 125 265, 200 x 100 (1.4 MiB) 248 440, 400 x 160 750 560).
+constexpr std::size_t kRingPopulations2 = std::size_t(3) << 19;
 constexpr std::size_t kSmallBytes2 = 65536;
 static_assert(8 * sizeof(double) + sizeof(orr::ForceScratch) <= kSmallBytes2);
 
@@ -183,11 +193,18 @@ void initialize2(orr_lbm2d* h, const double* rho, const double* ux, const double
         double* base = static_cast<double*>(h->f[1]);
         const double* src[3] = {rho, ux, uy};
         orr::HostSpan spans[3];
+        const bool ring = 3 * cells * sizeof(double) >= kRingFields2;
         for (int k = 0; k < 3; ++k) {
             staged[k] = base + static_cast<std::size_t>(k) * cells;
-            spans[k] = {const_cast<double*>(src[k]), staged[k], cells * 8};
+            spans[k] = {const_cast<double*>(src[k]), staged[k], cells * sizeof(double)};
+            if (!ring) {
+                check(cudaMemcpyAsync(staged[k], src[k], spans[k].bytes, cudaMemcpyHostToDevice, h->stream),
+                      "initial state upload");
+            }
         }
-        orr::copy_to_device(spans, 3, h->stream, h->device);
+        if (ring) {
+            orr::copy_to_device(spans, 3, h->stream, h->device);
+        }
     }
     const bool inflow = c.x_boundary == ORR_X_INFLOW_OUTFLOW;
     check(h->ops->init(h->g, h->cls, staged[0], staged[1], staged[2], inflow ? c.inlet_ux : 0.0,
@@ -419,7 +436,7 @@ orr_status orr_lbm2d_populations(orr_lbm2d* solver, double* f) {
             orr::copy_to_host(&all, 1, h->stream, h->device);
             return ORR_OK;
         }
-        if (h->storage == ORR_STORAGE_F32) {
+        if (h->storage == ORR_STORAGE_F32 && n * sizeof(double) >= kRingPopulations2) {
             orr::HostSpan spans[d2::Q];
             for (int i = 0; i < d2::Q; ++i) {
                 spans[i] = {f + i * cells, static_cast<float*>(h->f[h->cur]) + i * cells, cells * 4, true, d2::w(i)};
@@ -436,7 +453,11 @@ orr_status orr_lbm2d_populations(orr_lbm2d* solver, double* f) {
             for (std::size_t c = 0; c < cells; ++c) {
                 const std::size_t k = static_cast<std::size_t>(i) * cells + c;
                 double v;
-                if (h->storage == ORR_STORAGE_F16) {
+                if (h->storage == ORR_STORAGE_F32) {
+                    float x;
+                    std::memcpy(&x, raw.data() + 4 * k, 4);
+                    v = x;
+                } else if (h->storage == ORR_STORAGE_F16) {
                     __half x;
                     std::memcpy(&x, raw.data() + 2 * k, 2);
                     v = static_cast<double>(__half2float(x));
