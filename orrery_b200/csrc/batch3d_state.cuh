@@ -280,8 +280,9 @@ struct orr_batch3d {
 
     // One row-tile step of member m from buffer `from` on stream s.
     void member_step(orr_lbm3d* m, uint32_t from, cudaStream_t s) {
-        check(ops->step(m->g, m->phys(), m->f[from], m->f[1 - from], m->buffers(static_cast<int>(from)), smag, block,
-                        npt == 2 ? 2u : 1u, false, s),
+        StepBuffers3D b = m->buffers(static_cast<int>(from));
+        b.beside = branched() && members.size() > 1;
+        check(ops->step(m->g, m->phys(), m->f[from], m->f[1 - from], b, smag, block, npt == 2 ? 2u : 1u, false, s),
               "batch step kernel");
     }
 

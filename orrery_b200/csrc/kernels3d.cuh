@@ -676,6 +676,7 @@ struct StepBuffers3D {
     const uint32_t* wall_cell; // the boundary nodes (open lattices with interpolated walls)
     uint32_t wall_count;     // their number
     uint32_t wall_layers;    // grid layers of the wall list's blocks (set by the launcher)
+    uint32_t beside;         // other lattices' steps run beside this one (for the launcher)
     // Convective-outlet history (arithmetic type): a step from buffer k reads
     // hist[k] and writes hist[1 - k] (a lattice with one buffer passes it
     // twice).  In place, the rows that share a 32-byte sector of the history
@@ -1172,15 +1173,17 @@ __device__ __forceinline__ void wall_node3(const Geom3D& g, const Phys3D<typenam
 }
 
 // Resident 256-thread blocks per SM the row step is compiled for: 48
-// registers for the binary32 flat step, 40 for the flat step of the 2-byte
-// storages, 64 for the general one, 128 for binary64.  The flat step fits 48
-// without spills, and the extra resident warps hide more of the memory
-// latency: 45.5 against 42.8 GLUPS for binary16 storage in 128-thread blocks,
-// 41.4 against 39.9 for binary32 in 256-thread blocks (256 x 128 x 128 sphere
-// channel).  The 2-byte forms, which issue more instructions per byte moved,
-// gain again from 48 warps at 40 registers despite a few spilled values
-// (binary16 88.1 against 92.1 us per step, bfloat16 89.8 against 93.1);
-// binary32 loses there (105.2 against 101.1 us), so it keeps 48 registers.
+// registers for the binary32 forms of open lattices, 40 for those of the 2-byte
+// storages, 64 for the general one, 128 for binary64.  The binary32 form with
+// halfway walls fits 48 without spills, and the extra resident warps hide more
+// of the memory latency: 41.4 against 39.9 GLUPS in 256-thread blocks (256 x
+// 128 x 128 sphere channel); 40 registers lose (105.2 against 101.1 us per step).
+// The 2-byte forms issue more instructions per byte moved and gain from 48
+// warps at 40 registers despite spilled values (binary16 88.1 against 92.1 us at
+// 48 registers).  With halfway walls they step the lattices that the linear order
+// leaves to the rows (launcher's step_linear).  With interpolated walls every
+// form spills, the 2-byte ones 260 to 290 bytes of stores at 40 registers, which
+// lattices of one or two waves do not earn back (launcher's roomy_walls).
 template <class S, Walls kWalls>
 constexpr int kStepMinBlocks = sizeof(typename Storage<S>::A) == 8 ? 2
                                : kWalls == Walls::General      ? 4
@@ -1224,10 +1227,10 @@ inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, uint32_t block, 
 // of row (y, z).  b.hist[0] is the source buffer's history.
 // kWalls: Halfway for lattices with g.flat set, Interpolated for those with
 // g.open only, General for the others.
-// kDense: blocks of at most 128 threads, five of them an SM (96 registers instead
-// of 122), for binary64 with halfway walls (dense_rows in the launcher).
-template <class S, bool kSmag, Walls kWalls, bool kDense = false>
-__global__ void __launch_bounds__(kDense ? 128 : 256, kDense ? 5 : kStepMinBlocks<S, kWalls>)
+// kThreads, kBlocks: the largest block and the blocks an SM that the registers
+// leave room for (dense_rows and roomy_walls in the launcher name other pairs).
+template <class S, bool kSmag, Walls kWalls, int kThreads = 256, int kBlocks = kStepMinBlocks<S, kWalls>>
+__global__ void __launch_bounds__(kThreads, kBlocks)
     step3d_kernel(Geom3D g, Phys3D<typename Storage<S>::A> p, const S* src, S* __restrict__ dst, StepBuffers3D b) {
     uint32_t z = blockIdx.z;
     uint32_t lane = threadIdx.x;

@@ -54,16 +54,22 @@ template <class S> struct Launch3D {
             if (g.flat) {
                 if constexpr (sizeof(A) == 8) {
                     if (dense_rows(g, block)) {
-                        return launch_step<S>(&step3d_kernel<S, K, Walls::Halfway, true>, grid, block, chained, s, gg,
+                        return launch_step<S>(&step3d_kernel<S, K, Walls::Halfway, 128, 5>, grid, block, chained, s, gg,
                                               p, in, out, b);
                     }
                 }
                 return launch_step<S>(&step3d_kernel<S, K, Walls::Halfway>, grid, block, chained, s, gg, p, in, out, b);
             }
-            if (walls_listed(g, block, b.wall_count)) {
+            if (walls_listed(g, block, b.wall_count, b.beside != 0u)) {
                 StepBuffers3D w = b;
                 w.wall_layers = wall_layers(g, block, b.wall_count);
                 const dim3 with_walls(gg.tiles_x, g.ny, g.nz + w.wall_layers);
+                if constexpr (sizeof(S) == 2) {
+                    if (roomy_walls(g) && b.beside == 0u) {
+                        return launch_step<S>(&step3d_kernel<S, K, Walls::Interpolated, 256, 4>, with_walls, block,
+                                              chained, s, gg, p, in, out, w);
+                    }
+                }
                 return launch_step<S>(&step3d_kernel<S, K, Walls::Interpolated>, with_walls, block, chained, s, gg, p, in,
                                    out, w);
             }
@@ -80,10 +86,27 @@ template <class S> struct Launch3D {
 
     // Whether an open lattice's interpolated walls are stepped from their list.
     // The layers share the grid's z with the rows: a lattice whose nz leaves them no
-    // room takes the general node code.
-    static bool walls_listed(const Geom3D& g, uint32_t block, uint32_t wall_count) {
-        return g.open && !g.flat && uint64_t{g.nz} + wall_layers(g, block, wall_count) <= 65535u;
+    // room takes the general node code.  So do the storages with binary32
+    // arithmetic between 10,000 and 300,000 nodes, where one or two waves hold the
+    // grid and the list's chain adds to the rows' (its registers spill in every
+    // row), unless other lattices run beside this one (eight of 64 x 32 x 32, binary32
+    // 28.7 19.8).  us per step, general and listed (40 registers), binary16: 48 x 24 x 24
+    // 11.9 14.6, 64 x 32 x 32 12.0 16.6, 96 x 48 x 48 14.1 17.9; binary32 8.7 10.1, 9.6
+    // 10.0, 12.0 13.6; above and below, binary32: 5 x 4 x 3 6.0 3.3, 16 x 8 x 8 with the
+    // convective outlet 8.3 7.9, 112 x 56 x 56 15.6 15.2, 192 x 96 x 96 61 56.
+    static bool walls_listed(const Geom3D& g, uint32_t block, uint32_t wall_count, bool beside) {
+        if (!g.open || g.flat || uint64_t{g.nz} + wall_layers(g, block, wall_count) > 65535u) {
+            return false;
+        }
+        return sizeof(A) == 8 || wall_count == 0u || beside || g.cells < 10000u || g.cells >= 300000u;
     }
+
+    // Whether the listed form of a 2-byte storage is compiled for 64 registers
+    // (4 blocks an SM) or, where more warps pay for its spills, 40 (6).  us per step
+    // with 40 and 64: 24 x 12 x 12 13.6 11.4, 112 x 56 x 56 21.9 16.4, 128 x 64 x 64 22.8
+    // 16.6, 144 x 72 x 72 25.9 23.1, 160 x 80 x 80 (1.0 million nodes) 29.3 28.2, with
+    // sponge and convective outlet 31.5 32.4; 192 x 96 x 96 45.4 51.0.
+    static bool roomy_walls(const Geom3D& g) { return sizeof(S) == 2 && g.cells < 900000u; }
 
     // The binary64 step waits on memory and long arithmetic with 16 warps an SM;
     // 20 at 96 registers hide more of both for some spilled values: us per
@@ -177,15 +200,21 @@ template <class S> struct Launch3D {
         }
         if constexpr (sizeof(A) == 8) {
             if (dense_rows(g, block)) {
-                return registers(smag ? &step3d_kernel<S, true, Walls::Halfway, true>
-                                      : &step3d_kernel<S, false, Walls::Halfway, true>);
+                return registers(smag ? &step3d_kernel<S, true, Walls::Halfway, 128, 5>
+                                      : &step3d_kernel<S, false, Walls::Halfway, 128, 5>);
+            }
+        }
+        if constexpr (sizeof(S) == 2) {
+            if (walls_listed(g, block, wall_count, false) && roomy_walls(g)) {
+                return registers(smag ? &step3d_kernel<S, true, Walls::Interpolated, 256, 4>
+                                      : &step3d_kernel<S, false, Walls::Interpolated, 256, 4>);
             }
         }
         const auto of = [&]<Walls K>() {
             return registers(smag ? &step3d_kernel<S, true, K> : &step3d_kernel<S, false, K>);
         };
         return g.flat                                ? of.template operator()<Walls::Halfway>()
-               : walls_listed(g, block, wall_count) ? of.template operator()<Walls::Interpolated>()
+               : walls_listed(g, block, wall_count, false) ? of.template operator()<Walls::Interpolated>()
                                                      : of.template operator()<Walls::General>();
     }
 
