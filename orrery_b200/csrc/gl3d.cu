@@ -326,7 +326,7 @@ orr_status orr_gl3d_step(orr_gl3d* tables, const orr_gl3d_params* params, const 
         b.hist[0] = b.hist[1] = outlet;   // the driver's one buffer, updated in place
         b.inlet = t->inlet;
         const bool smag = params->smagorinsky_c2 > 0.0f;
-        const uint32_t block = ops3d_f32().step_linear(t->g) ? linear_block(t->g.cells)
+        const uint32_t block = ops3d_f32().step_linear(t->g, linear_block(t->g.cells)) ? linear_block(t->g.cells)
                                : params->nx % 256 == 0       ? 256u
                                                              : 128u;
         check(ops3d_f32().step(t->g, &phys, src, dst, b, smag, block, 1, false, s), "gl3d step kernel");

@@ -63,8 +63,9 @@ struct Ops3D {
                          double* result, const uint32_t* status, cudaStream_t s);
     cudaError_t (*mass)(const Geom3D& g, const uint8_t* cls, const void* f, double* out,
                         cudaStream_t s);
-    // Whether the one-node step of lattice g runs in linear order.
-    bool (*step_linear)(const Geom3D& g);
+    // Whether the one-node step of lattice g in blocks of `block` threads runs in
+    // linear order.
+    bool (*step_linear)(const Geom3D& g, uint32_t block);
     // Registers per thread of lattice g's step kernel (wall_count: StepBuffers3D's).
     int (*step_registers)(const Geom3D& g, bool smag, uint32_t block, uint32_t npt, uint32_t wall_count);
     // Whether the pair step serves lattice g with blocks of `block` threads

@@ -35,7 +35,7 @@ template <class S> struct Launch3D {
             }
         }
         if constexpr (sizeof(A) == 4) {
-            if (step_linear(g)) {
+            if (step_linear(g, block)) {
                 LinearOffsets3D l;
                 for (int i = 0; i < d3::Q; ++i) {
                     const int64_t to = static_cast<int64_t>(i) * static_cast<int64_t>(g.cells);
@@ -120,12 +120,21 @@ template <class S> struct Launch3D {
     }
 
     // The linear order serves flat lattices whose buffers 32-bit byte offsets
-    // reach.  The 2-byte storages gain from it at every size; binary32, bound
-    // by memory, where rows do not fill their tiles (337 x 193 x 193 334 -> 324
-    // us per step) and not where they do (256 x 128 x 128 102.9 -> 104.5).
-    static bool step_linear(const Geom3D& g) {
-        return sizeof(A) == 4 && g.flat && d3::Q * g.cells * sizeof(S) <= 0xffffffffull &&
-               (sizeof(S) == 2 || g.nx % 64 != 0);
+    // reach.  us per step, rows and linear:
+    // The 2-byte storages gain from it (binary16 256 x 128 x 128 88 79, 337 x 193 x
+    // 193 268 231) except in blocks of at most 128 threads beyond 30 million nodes
+    // (128 threads, 480 x 240 x 240 567 560, 512 x 256 x 256 650 674).
+    // Binary32 is bound by memory.  It gains where nx is not a multiple of 64 (66 x
+    // 120 x 120 35.5 27.9, 337 x 120 x 120 134 120, 200 x 200 x 200 199 192; multiples
+    // of 8 gain less and a few lose: 120 x 120 x 120 45.2 46.3, 160 59.4 60.0, 280
+    // 99.3 101.0, 250 x 125 x 125 107 109), not where it is (256 x 128 x 128 102.9 104.5), and
+    // not in one wave of row tiles (40 x 20 x 20 3.46 4.10, 56 x 28 x 28 4.48 5.01;
+    // 72 x 36 x 36 5.25 5.33, with 64 threads 6.79 5.63; 80 x 40 x 40 7.05 5.78).
+    static bool step_linear(const Geom3D& g, uint32_t block) {
+        if (sizeof(A) != 4 || !g.flat || d3::Q * g.cells * sizeof(S) > 0xffffffffull) {
+            return false;
+        }
+        return sizeof(S) == 2 ? block > 128u || g.cells < 30000000u : g.nx % 64 != 0 && g.cells >= 60000u;
     }
 
     static auto linear_kernel(bool smag) {
@@ -194,7 +203,7 @@ template <class S> struct Launch3D {
             }
         }
         if constexpr (sizeof(A) == 4) {
-            if (step_linear(g)) {
+            if (step_linear(g, block)) {
                 return registers(linear_kernel(smag));
             }
         }

@@ -466,7 +466,7 @@ orr_status orr_lbm3d_create(const orr_lbm3d_config* config, const uint8_t* solid
                                                "and blocks of at most 128 threads"};
             }
             h->row_npt = 2;
-        } else if (o.block_x == 0 && h->ops->step_linear(g)) {
+        } else if (o.block_x == 0 && h->ops->step_linear(g, linear_block(g.cells))) {
             h->block = linear_block(g.cells);
         } else if (o.block_x == 0 && !binary32 && g.open && one_warp_rows(g.nx, g.ny, g.nz)) {
             h->block = 32u;
@@ -765,7 +765,7 @@ orr_status orr_lbm3d_kernel_info(const orr_lbm3d* solver, orr_kernel_info* info)
             k.block = solver->block;
             const uint32_t span = solver->block * solver->row_npt;
             k.nodes_per_thread = solver->row_npt;
-            k.grid = solver->row_npt == 1 && solver->ops->step_linear(solver->g)
+            k.grid = solver->row_npt == 1 && solver->ops->step_linear(solver->g, solver->block)
                          ? static_cast<uint32_t>((solver->g.cells + span - 1) / span)
                          : ((solver->g.nx + span - 1) / span) * solver->g.ny * solver->g.nz;
             k.registers = solver->ops->step_registers(solver->g, solver->smag, solver->block, solver->row_npt,
