@@ -190,6 +190,7 @@ orr_status orr_batch3d_set_schedule(orr_batch3d* batch, const orr_batch_schedule
         }
         b->kernel = s.kernel;
         b->block = s.block;
+        b->named = true;
         b->stages = s.kernel == ORR_KERNEL_STAGED ? s.stages : 0;
         b->npt = s.nodes_per_thread;
         b->branches = s.branches;
@@ -297,6 +298,7 @@ orr_status orr_batch3d_tune(orr_batch3d* batch, uint32_t graphs_per_trial, orr_b
             }
             b->kernel = c.kernel;
             b->block = c.block;
+            b->named = true;
             b->stages = c.stages;
             b->npt = c.npt;
             b->branches = c.branches;

@@ -33,6 +33,7 @@ inline constexpr Candidate kCandidates[] = {
     {ORR_KERNEL_ROWS, 128, 0, 0, 0},    {ORR_KERNEL_ROWS, 128, 0, 0, 64},
     {ORR_KERNEL_ROWS, 128, 0, 2, 0},    {ORR_KERNEL_ROWS, 128, 0, 2, 64},
     {ORR_KERNEL_ROWS, 64, 0, 0, 0},     {ORR_KERNEL_ROWS, 64, 0, 0, 64},
+    {ORR_KERNEL_ROWS, 256, 0, 0, 0},    {ORR_KERNEL_ROWS, 256, 0, 0, 64},
 };
 
 } // namespace orr
@@ -55,6 +56,7 @@ struct orr_batch3d {
     uint32_t npt = 0;         // nodes per thread of a staged span (0: the storage's default),
                               // or of the row-tile step (2: the pair step where it serves a member)
     uint32_t branches = 0;    // 0: one stream; else members spread over this many graph branches
+    bool named = true;        // the caller named the block (else members in linear order take their own)
     StagedShape shape{};
 
     // Branched schedule: member k runs its own single-lattice launches (its
@@ -280,9 +282,11 @@ struct orr_batch3d {
 
     // One row-tile step of member m from buffer `from` on stream s.
     void member_step(orr_lbm3d* m, uint32_t from, cudaStream_t s) {
+        const bool linear = ops->step_linear(m->g, named ? block : linear_block(m->g.cells));
+        const uint32_t width = row_block(block, named, linear, m->g.cells);
         StepBuffers3D b = m->buffers(static_cast<int>(from));
         b.beside = branched() && members.size() > 1;
-        check(ops->step(m->g, m->phys(), m->f[from], m->f[1 - from], b, smag, block, npt == 2 ? 2u : 1u, false, s),
+        check(ops->step(m->g, m->phys(), m->f[from], m->f[1 - from], b, smag, width, npt == 2 ? 2u : 1u, false, s),
               "batch step kernel");
     }
 

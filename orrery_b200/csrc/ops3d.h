@@ -24,6 +24,12 @@ struct ForceScratch;
 // 382 379; 512 x 256 x 256 692 589 (binary16).
 inline uint32_t linear_block(uint64_t cells) { return cells >= 5500000u ? 256u : 128u; }
 
+// Block of a batch member's row step: the schedule's, or the member's own where it
+// runs in linear order and nobody named one.
+inline uint32_t row_block(uint32_t block, bool named, bool linear, uint64_t cells) {
+    return linear && !named ? linear_block(cells) : block;
+}
+
 // Whether the binary64 row step of an open lattice takes one-warp blocks where
 // the caller names none.  Its blocks are limited by registers (16 or 20 warps an
 // SM; the figures are with 16), and the warps of a 128-node tile beyond the row's

@@ -497,6 +497,7 @@ struct orr_server {
             if (orr_batch3d_set_schedule(batch, &sched) != ORR_OK) {
                 throw Refusal{ORR_ERR_INVALID, orr_batch3d_last_error(batch)};
             }
+            batch->named = opt.block != 0;
             uint32_t counters[kServeCounters] = {0, 0};
             for (;;) {
                 {
