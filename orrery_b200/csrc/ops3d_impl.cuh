@@ -109,13 +109,15 @@ template <class S> struct Launch3D {
     static bool roomy_walls(const Geom3D& g) { return sizeof(S) == 2 && g.cells < 900000u; }
 
     // The binary64 step waits on memory and long arithmetic with 16 warps an SM;
-    // 20 at 96 registers hide more of both for some spilled values: us per
-    // step with the convective outlet, 256 x 128 x 128 274 -> 259, 128 x 64 x 64 44.4 -> 41.4, 337 x 193 x 193 780 -> 765.
-    // Where 16 warps an SM hold the lattice the spills are all that changes
-    // (64 x 32 x 32 8.1 -> 8.4), interpolated walls spill far more (337 x 193 x 193
-    // 806 -> 827), and 24 warps at 80 registers are slower (256 x 128 x 128 305).
+    // 20 at 96 registers hide more of both for some spilled values.  us per step
+    // without and with: 64 x 48 x 48 14.1 13.7, 97 x 65 x 65 37.0 34.9, 128 x 64 x 64 37.9
+    // 35.2, 256 x 128 x 128 239 228 (convective outlet 259 247).  Where 16 warps an SM
+    // hold the lattice the spills are all that changes (64 x 32 x 32 8.1 8.4), larger
+    // lattices are bound by memory (300 x 150 x 150 396 403, 337 x 193 x 193 744 766),
+    // interpolated walls spill far more (337 x 193 x 193 806 827), and 24 warps at 80
+    // registers are slower (256 x 128 x 128 305).
     static bool dense_rows(const Geom3D& g, uint32_t block) {
-        return sizeof(A) == 8 && g.flat && block <= 128 &&
+        return sizeof(A) == 8 && g.flat && block <= 128 && g.cells < 6000000u &&
                static_cast<uint64_t>((g.nx + 31) / 32) * g.ny * g.nz > 148u * 16u;
     }
 
