@@ -1194,9 +1194,13 @@ constexpr int kStepMinBlocks = sizeof(typename Storage<S>::A) == 8 ? 2
 // `chained`) a launch is set up while the step before it ends: it touches no
 // population or history before this wait, which returns when that step has
 // completed and its writes are visible.  Nothing happens in a launch that is not
-// chained.  `index` enters every address of the buffers that steps write, which
-// pins those accesses behind the wait; `src` is not __restrict__ in these
-// kernels so that its loads are not read-only ones.  Bound: small lattices are
+// chained.  The asm's memory clobber keeps every access to the buffers that
+// steps write behind the wait; `index`, which enters the populations' addresses
+// (the outlet history's come from y and z), ties them to it as operands too.
+// `src` is not __restrict__ in these kernels so that its loads are not read-only
+// ones; in the functions they call it is: from there to the kernel's end nothing
+// writes that buffer (without it the binary32 form with halfway walls and the
+// closure spills 8 bytes at its 48 registers).  Bound: small lattices are
 // launch latency.  us per step, not chained -> chained: 64 x 32 x 32 4.39 ->
 // 4.23, 400 x 160 3.59 -> 3.34.  Letting the next step's blocks in early
 // (launch_dependents after the wait) takes 1% off 128^3 but places waiting
