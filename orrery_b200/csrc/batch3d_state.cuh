@@ -285,7 +285,7 @@ struct orr_batch3d {
         const bool linear = ops->step_linear(m->g, named ? block : linear_block(m->g.cells));
         const uint32_t width = row_block(block, named, linear, m->g.cells);
         StepBuffers3D b = m->buffers(static_cast<int>(from));
-        b.beside = branched() && members.size() > 1;
+        b.wall_layers = branched() && members.size() > 1 ? kBeside : 0u;
         check(ops->step(m->g, m->phys(), m->f[from], m->f[1 - from], b, smag, width, npt == 2 ? 2u : 1u, false, s),
               "batch step kernel");
     }

@@ -668,6 +668,8 @@ __device__ __forceinline__ void inlet_west3(A (&f)[d3::Q], const A* inlet) {
 
 // ------------------------------------------------------------------- step --
 
+constexpr uint32_t kBeside = ~0u;
+
 struct StepBuffers3D {
     const uint8_t* cls;      // node classes
     const uint32_t* nmask;   // per node, bit i: direction i bounces back (solid source)
@@ -675,8 +677,10 @@ struct StepBuffers3D {
     const void* wall_q;      // 19 fractions per slot (arithmetic type)
     const uint32_t* wall_cell; // the boundary nodes (open lattices with interpolated walls)
     uint32_t wall_count;     // their number
-    uint32_t wall_layers;    // grid layers of the wall list's blocks (set by the launcher)
-    uint32_t beside;         // other lattices' steps run beside this one (for the launcher)
+    // Grid layers of the wall list's blocks, set by the launcher; its caller sets
+    // kBeside where other lattices' steps run beside this one.  (A field of its own
+    // moved the kernels' parameters and cost the binary16 linear step 5%.)
+    uint32_t wall_layers;
     // Convective-outlet history (arithmetic type): a step from buffer k reads
     // hist[k] and writes hist[1 - k] (a lattice with one buffer passes it
     // twice).  In place, the rows that share a 32-byte sector of the history

@@ -50,6 +50,7 @@ template <class S> struct Launch3D {
             }
         }
         const dim3 grid(gg.tiles_x, g.ny, g.nz);
+        const bool beside = b.wall_layers == kBeside;
         const auto launch = [&]<bool K>() {
             if (g.flat) {
                 if constexpr (sizeof(A) == 8) {
@@ -60,12 +61,12 @@ template <class S> struct Launch3D {
                 }
                 return launch_step<S>(&step3d_kernel<S, K, Walls::Halfway>, grid, block, chained, s, gg, p, in, out, b);
             }
-            if (walls_listed(g, block, b.wall_count, b.beside != 0u)) {
+            if (walls_listed(g, block, b.wall_count, beside)) {
                 StepBuffers3D w = b;
                 w.wall_layers = wall_layers(g, block, b.wall_count);
                 const dim3 with_walls(gg.tiles_x, g.ny, g.nz + w.wall_layers);
                 if constexpr (sizeof(S) == 2) {
-                    if (roomy_walls(g) && b.beside == 0u) {
+                    if (roomy_walls(g) && !beside) {
                         return launch_step<S>(&step3d_kernel<S, K, Walls::Interpolated, 256, 4>, with_walls, block,
                                               chained, s, gg, p, in, out, w);
                     }
