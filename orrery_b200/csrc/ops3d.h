@@ -72,6 +72,8 @@ struct Ops3D {
     // Whether the one-node step of lattice g in blocks of `block` threads runs in
     // linear order.
     bool (*step_linear)(const Geom3D& g, uint32_t block);
+    // Blocks of lattice g's step kernel (wall_count: StepBuffers3D's).
+    uint32_t (*step_grid)(const Geom3D& g, uint32_t block, uint32_t npt, uint32_t wall_count);
     // Registers per thread of lattice g's step kernel (wall_count: StepBuffers3D's).
     int (*step_registers)(const Geom3D& g, bool smag, uint32_t block, uint32_t npt, uint32_t wall_count);
     // Whether the pair step serves lattice g with blocks of `block` threads

@@ -195,6 +195,14 @@ template <class S> struct Launch3D {
         return sizeof(S) == 2 && g.flat && g.nx % 2 == 0 && block % 32 == 0 && block <= 128;
     }
 
+    static uint32_t step_grid(const Geom3D& g, uint32_t block, uint32_t npt, uint32_t wall_count) {
+        if (npt == 1 && step_linear(g, block)) {
+            return static_cast<uint32_t>((g.cells + block - 1) / block);
+        }
+        const uint32_t layers = walls_listed(g, block, wall_count, false) ? wall_layers(g, block, wall_count) : 0u;
+        return (g.nx + block * npt - 1) / (block * npt) * g.ny * (g.nz + layers);
+    }
+
     static int step_registers(const Geom3D& g, bool smag, uint32_t block, uint32_t npt, uint32_t wall_count) {
         cudaFuncAttributes a{};
         const auto registers = [&a](auto kernel) {
@@ -395,7 +403,7 @@ template <class S> struct Launch3D {
 
     static const Ops3D& table() {
         static const Ops3D ops{&step,   &init,   &history,        &moments,          &force,
-                               &mass,   &step_linear, &step_registers, &pairs_ok, &staged, &staged_occupancy,
+                               &mass,   &step_linear, &step_grid, &step_registers, &pairs_ok, &staged, &staged_occupancy,
                                &staged_smem, &staged_registers, &tiled, &tiled_occupancy,
                                &tiled_registers, &force_batch};
         return ops;

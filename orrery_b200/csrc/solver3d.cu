@@ -763,11 +763,8 @@ orr_status orr_lbm3d_kernel_info(const orr_lbm3d* solver, orr_kernel_info* info)
         } else {
             k.kernel = ORR_KERNEL_ROWS;
             k.block = solver->block;
-            const uint32_t span = solver->block * solver->row_npt;
             k.nodes_per_thread = solver->row_npt;
-            k.grid = solver->row_npt == 1 && solver->ops->step_linear(solver->g, solver->block)
-                         ? static_cast<uint32_t>((solver->g.cells + span - 1) / span)
-                         : ((solver->g.nx + span - 1) / span) * solver->g.ny * solver->g.nz;
+            k.grid = solver->ops->step_grid(solver->g, solver->block, solver->row_npt, solver->wall_count);
             k.registers = solver->ops->step_registers(solver->g, solver->smag, solver->block, solver->row_npt,
                                                       solver->wall_count);
         }
