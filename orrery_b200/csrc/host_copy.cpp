@@ -28,7 +28,7 @@ namespace {
 constexpr std::size_t kChunk = std::size_t(4) << 20;
 constexpr int kSlots = 8;
 constexpr int kMaxWorkers = 16;
-constexpr std::size_t kAloneBytes = std::size_t(3) << 19;
+constexpr std::size_t kAloneBytes = std::size_t(1) << 20;
 constexpr std::size_t kThreadBytes = std::size_t(512) << 10;
 
 // One staged copy at a time in the process: the ring is shared.  It is
@@ -154,9 +154,9 @@ void staged(bool upload, const std::vector<Chunk>& chunks, cudaStream_t stream, 
     // memory and 10 from its own: this thread up to kAloneBytes of host memory, then
     // one for each kThreadBytes, up to worker_count (so only widening read-backs
     // below 8 MiB take fewer).  us per read-back of the fields with one thread (own
-    // and other node) and sixteen: 16 x 8 x 8 40 380, 40 x 20 x 20 (0.5 MiB) 65 150 400,
-    // 56 x 28 x 28 140 360 420, 64 x 32 x 32 (2 MiB) 200 515 450, 80 x 40 x 40 360 960
-    // 500; with one per 0.5 MiB the last two 170 to 185 and 300 to 330 on its own node.
+    // and other node), one per 0.5 MiB, and sixteen: 16 x 8 x 8 40, 40, and 380, 40 x 20 x 20
+    // (0.5 MiB) 65, 150, and 400, 400 x 160 (1.5 MiB) 150 385 200 420, 64 x 32 x 32 (2 MiB)
+    // 200 515 170 to 310 450, 80 x 40 x 40 360 960 300 to 390 500.
     std::size_t host_bytes = 0;
     for (const Chunk& c : chunks) {
         host_bytes += c.widen ? 2 * c.len : c.len;

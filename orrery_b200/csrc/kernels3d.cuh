@@ -1637,11 +1637,11 @@ __device__ __forceinline__ bool add_link3(uint64_t nx, uint64_t plane, uint64_t 
     return true;
 }
 
-// Blocks of the solvers' force kernels, at most: eight per SM, all the threads
-// it holds, since the links' loads are a chain of two round trips.  us per call
-// with two per SM and eight, binary32: 4.4 million links 106 80, 16.7 million 346
-// 217; D2Q9, 1.3 million solids of 4096 x 4096 277 116 (up to 1.2 million links
-// the two take the same).
+// Blocks of the solvers' force kernels, at most: eight per SM, twice what its
+// registers hold of the 3D one at a time, since the links' loads are a chain of two
+// round trips.  us per call with two per SM and eight, binary32: 4.4 million links
+// 106 80, 16.7 million 346 217; D2Q9, 1.3 million solids of 4096 x 4096 277 116 (up
+// to 1.2 million links the two take the same).
 constexpr uint32_t kForceBlocks = 1184;
 constexpr uint32_t kForceThreads = 256;
 
