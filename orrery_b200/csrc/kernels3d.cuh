@@ -1283,7 +1283,7 @@ template <class S, class O> __device__ __forceinline__ S* bytes_from(S* p, O n) 
 // the buffer for every node: direction i's plane has i planes below it and
 // 18 - i above), and one 32-bit byte offset per access is added to the two
 // buffers' bases (a buffer is below 4 GB).  Bound: instruction issue for the
-// 2-byte storages (82% of the slots), memory for binary32.  Against the row
+// 2-byte storages (81% of the slots), memory for binary32.  Against the row
 // tiles, us per step: binary16 256 x 128 x 128 89.0 -> 79.3, 128 x 110 x 105 40.1
 // -> 34.5, 512 x 256 x 256 640 -> 566, 337 x 193 x 193 268 -> 230; binary32
 // 337 x 193 x 193 334 -> 324, but 256 x 128 x 128 102.9 -> 104.5 (the

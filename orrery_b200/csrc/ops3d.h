@@ -38,7 +38,9 @@ inline uint32_t row_block(uint32_t block, bool named, bool linear, uint64_t cell
 // are short and leave one warp idle.  us per step with 128 and 32 nodes, halfway
 // walls: nx 64 10.3 8.1, 160 85.0 76.3, 200 158 145, 300 471 426, 337 634 590 (ny =
 // nz = nx / 2); not taken: 40 6.3 6.6, 80 14.7 14.7 (interpolated walls 14.9 15.2),
-// 97 21.8 24.0, 128 x 64 x 64 38.3 39.3.
+// 97 21.8 24.0, 128 x 64 x 64 38.3 39.3.  The line stands with the 96-register form
+// too (5 tiles an SM): 300 x 14 x 14 (588 tiles) 6.9 7.2, 160 x 18 x 18 (648) 8.7 7.0, 300 x
+// 15 x 15 (675) 8.4 7.3, 300 x 16 x 16 (768) 8.5 7.7.
 inline bool one_warp_rows(uint64_t nx, uint64_t ny, uint64_t nz) {
     const uint64_t idle = (4u - (nx + 31u) / 32u % 4u) % 4u;   // warps of the last tile
     return (nx > 128u ? idle > 0u : idle >= 2u) && (nx + 127u) / 128u * ny * nz > 4u * 148u;
