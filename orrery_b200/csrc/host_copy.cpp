@@ -14,6 +14,7 @@
 #include "host_copy.h"
 
 #include <algorithm>
+#include <atomic>
 #include <condition_variable>
 #include <cstring>
 #include <mutex>
@@ -28,7 +29,7 @@ namespace {
 constexpr std::size_t kChunk = std::size_t(4) << 20;
 constexpr int kSlots = 8;
 constexpr int kMaxWorkers = 16;
-constexpr std::size_t kAloneBytes = std::size_t(1) << 20;
+constexpr std::size_t kAloneBytes = std::size_t(2) << 20;
 constexpr std::size_t kThreadBytes = std::size_t(512) << 10;
 
 // One staged copy at a time in the process: the ring is shared.  It is
@@ -150,13 +151,14 @@ void staged(bool upload, const std::vector<Chunk>& chunks, cudaStream_t stream, 
     }
     Events ev;
     const std::size_t n = chunks.size();
-    // A thread takes about 25 us to start and moves 4 GB/s from another NUMA node's
-    // memory and 10 from its own: this thread up to kAloneBytes of host memory, then
-    // one for each kThreadBytes, up to worker_count (so only widening read-backs
-    // below 8 MiB take fewer).  us per read-back of the fields with one thread (own
-    // and other node), one per 0.5 MiB, and sixteen: 16 x 8 x 8 40, 40, and 380, 40 x 20 x 20
-    // (0.5 MiB) 65, 150, and 400, 400 x 160 (1.5 MiB) 150 385 200 420, 64 x 32 x 32 (2 MiB)
-    // 200 515 170 to 310 450, 80 x 40 x 40 360 960 300 to 390 500.
+    // One thread moves the fields at 10 GB/s in some processes and at 4 in others (the
+    // cause is not known), and threads take 100 us and more to start after a run: this
+    // thread up to kAloneBytes of host memory, then one for each kThreadBytes, up to
+    // worker_count (so only widening read-backs below 8 MiB take fewer).  us per
+    // read-back of the fields after 200 steps with one thread (the two kinds of
+    // process), one per 0.5 MiB, and sixteen: 48 x 24 x 24 (0.8 MiB) 95 to 240, 180, 485;
+    // 64 x 32 x 32 (2 MiB) 190 to 515, 350, 495; 72 x 36 x 36 250 to 710, 380 to 410, 540;
+    // 80 x 40 x 40 (3.9 MiB) 315 to 960, 420 to 515, 595.
     std::size_t host_bytes = 0;
     for (const Chunk& c : chunks) {
         host_bytes += c.widen ? 2 * c.len : c.len;
@@ -167,16 +169,49 @@ void staged(bool upload, const std::vector<Chunk>& chunks, cudaStream_t stream, 
     pr.filled.assign(n, 0);
     const auto slot = [&](std::size_t j) { return slots + (j % kSlots) * kChunk; };
 
+    // Waits for chunk j of a read-back and copies stripe t of it out of its slot.
+    const auto take_out = [&](std::size_t j, int t) {
+        if (!pr.wait([&] { return pr.posted > j; })) {
+            return false;
+        }
+        const cudaError_t s = cudaEventSynchronize(ev.e[j % kSlots]);
+        if (s != cudaSuccess) {
+            pr.fail(s, "staged read-back");
+            return false;
+        }
+        std::size_t a = 0, b = 0;
+        stripe(chunks[j].len, t, nworkers, a, b);
+        if (chunks[j].widen) {
+            widen_stripe(chunks[j], slot(j), a, b);
+        } else {
+            std::memcpy(chunks[j].host + a, slot(j) + a, b - a);
+        }
+        return true;
+    };
+    // Of a read-back whose chunks all fit the ring, this thread is a worker too
+    // once it has queued them, and each takes the next stripe that nobody has: the
+    // copy does not wait for a thread that starts late.
+    const bool shared = !upload && n <= static_cast<std::size_t>(kSlots);
+    std::atomic<std::size_t> next{0};
+
     auto worker = [&](int t) {
         const cudaError_t e = cudaSetDevice(device);
         if (e != cudaSuccess) {
             pr.fail(e, "cudaSetDevice");
             return;
         }
+        if (shared) {
+            for (std::size_t k = next++; k < n * static_cast<std::size_t>(nworkers); k = next++) {
+                if (!take_out(k / nworkers, static_cast<int>(k % nworkers))) {
+                    return;
+                }
+            }
+            return;
+        }
         for (std::size_t j = 0; j < n; ++j) {
-            std::size_t a = 0, b = 0;
-            stripe(chunks[j].len, t, nworkers, a, b);
             if (upload) {
+                std::size_t a = 0, b = 0;
+                stripe(chunks[j].len, t, nworkers, a, b);
                 // The slot is free once the DMA of chunk j - kSlots is done.
                 if (j >= static_cast<std::size_t>(kSlots)) {
                     if (!pr.wait([&] { return pr.posted > j - kSlots; })) {
@@ -189,32 +224,17 @@ void staged(bool upload, const std::vector<Chunk>& chunks, cudaStream_t stream, 
                     }
                 }
                 std::memcpy(slot(j) + a, chunks[j].host + a, b - a);
-            } else {
-                if (!pr.wait([&] { return pr.posted > j; })) {
-                    return;
-                }
-                const cudaError_t s = cudaEventSynchronize(ev.e[j % kSlots]);
-                if (s != cudaSuccess) {
-                    pr.fail(s, "staged read-back");
-                    return;
-                }
-                if (chunks[j].widen) {
-                    widen_stripe(chunks[j], slot(j), a, b);
-                } else {
-                    std::memcpy(chunks[j].host + a, slot(j) + a, b - a);
-                }
+            } else if (!take_out(j, t)) {
+                return;
             }
             pr.mark_filled(j);
         }
     };
 
-    // One worker whose chunks all fit the ring: this thread, after it has
-    // queued them.
-    const bool alone = !upload && nworkers == 1 && n <= static_cast<std::size_t>(kSlots);
     std::vector<std::thread> threads;
     threads.reserve(nworkers);
     try {
-        for (int t = 0; t < nworkers && !alone; ++t) {
+        for (int t = shared ? 1 : 0; t < nworkers; ++t) {
             threads.emplace_back(worker, t);
         }
         if (!upload) {
@@ -247,7 +267,7 @@ void staged(bool upload, const std::vector<Chunk>& chunks, cudaStream_t stream, 
         }
         pr.post(j);
     }
-    if (alone) {
+    if (shared) {
         worker(0);
     }
     for (auto& th : threads) th.join();
